@@ -44,7 +44,13 @@ struct FftPlan {
     int ntab;                 // float2 entries in `tab`
     const float2 *tw;         // device, n entries: exp(-2 pi i m / n)
     const float2 *tab;        // device, per generic stage R entries: exp(-2 pi i m / R)
+    // 678 and 478 (fft_pfa.cuh; NULL otherwise): index tables, and the
+    // transformed Rader sequence of the forward, then the inverse transform
+    const int *pfa_idx;
+    const float2 *pfa_h;
 };
+// entries of a thread's row in the index tables: 16-byte rows of v ints
+__device__ __host__ constexpr int pfa_ipad(int v) { return (v + 3) & ~3; }
 
 // element e of line l in a CTA's line buffer (see the layout note above)
 __device__ __forceinline__ int sidx(int e, int l, int nl) { return e * nl + (l ^ (e & (nl - 1))); }

@@ -85,6 +85,52 @@ void rader_tables(int R, int g, std::vector<float2> &tab) {
             tab.push_back(make_float2((float)cos(a), (float)sin(a)));
         }
 }
+// Tables of the prime-factor transform of N = C R, R - 1 = N1 N2 (fft_pfa.cuh,
+// g a primitive root mod R).  idx: per q1 the input places of (n1, q2), per q1
+// the output places of (k1, q2), in rows of pfa_ipad(C N2); then the C inputs
+// with n2 = 0 and the C outputs with k2 = 0 in rows of 8.  h: per direction
+// [a2][a1], the N1 x N2 transform of exp(-+2 pi i g^s / R) / (R - 1) placed at
+// (s mod N1, s mod N2).
+void pfa_tables(int R, int C, int N1, int N2, int g, std::vector<int> &idx, std::vector<float2> &h) {
+    const int N = C * R, M = R - 1, pad = pfa_ipad(C * N2);
+    std::vector<int> gp(M), gi(M), at(M);  // g^q, g^-q, and q from (q mod N1, q mod N2)
+    gp[0] = 1;
+    for (int q = 1; q < M; ++q) gp[q] = gp[q - 1] * g % R;
+    for (int q = 0; q < M; ++q) {
+        gi[q] = gp[(M - q) % M];
+        at[(q % N1) * N2 + q % N2] = q;
+    }
+    // k with k = a (mod C), b (mod R)
+    auto crt = [&](int a, int b) {
+        int k = b;
+        while (k % C != a) k += R;
+        return k;
+    };
+    idx.assign((size_t)2 * N1 * pad + 16, 0);
+    for (int q1 = 0; q1 < N1; ++q1)
+        for (int c = 0; c < C; ++c)
+            for (int q2 = 0; q2 < N2; ++q2) {
+                const int q = at[q1 * N2 + q2];
+                idx[q1 * pad + c * N2 + q2] = (R * c + C * gi[q]) % N;
+                idx[(N1 + q1) * pad + c * N2 + q2] = crt(c, gp[q]);
+            }
+    for (int c = 0; c < C; ++c) {
+        idx[2 * N1 * pad + c] = R * c % N;
+        idx[2 * N1 * pad + 8 + c] = crt(c, 0);
+    }
+    for (int dir = 0; dir < 2; ++dir)
+        for (int a2 = 0; a2 < N2; ++a2)
+            for (int a1 = 0; a1 < N1; ++a1) {
+                double re = 0.0, im = 0.0;
+                for (int s = 0; s < M; ++s) {
+                    const double w = (dir ? 2.0 : -2.0) * M_PI * gp[s] / R;
+                    const double t = -2.0 * M_PI * ((double)(s % N1 * a1 % N1) / N1 + (double)(s % N2 * a2 % N2) / N2);
+                    re += cos(w + t);
+                    im += sin(w + t);
+                }
+                h.push_back(make_float2((float)(re / M), (float)(im / M)));
+            }
+}
 }  // namespace
 
 int mm_fft_plan_get(int n, FftPlan *out) {
@@ -160,6 +206,22 @@ int mm_fft_plan_get(int n, FftPlan *out) {
     MM_CUDA_TRY(cudaMemcpy(d_tab, tab.data(), sizeof(float2) * tab.size(), cudaMemcpyHostToDevice));
     P.tw = d_tw;
     P.tab = d_tab;
+    if (n == 678 || n == 478) {
+        std::vector<int> idx;
+        std::vector<float2> h;
+        if (n == 678)
+            pfa_tables(113, 6, 16, 7, 3, idx, h);
+        else
+            pfa_tables(239, 2, 14, 17, 7, idx, h);
+        int *d_idx = nullptr;
+        float2 *d_h = nullptr;
+        MM_CUDA_TRY(cudaMalloc(&d_idx, sizeof(int) * idx.size()));
+        MM_CUDA_TRY(cudaMalloc(&d_h, sizeof(float2) * h.size()));
+        MM_CUDA_TRY(cudaMemcpy(d_idx, idx.data(), sizeof(int) * idx.size(), cudaMemcpyHostToDevice));
+        MM_CUDA_TRY(cudaMemcpy(d_h, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice));
+        P.pfa_idx = d_idx;
+        P.pfa_h = d_h;
+    }
     g_plans[{dev, n}] = P;
     *out = P;
     return MM_OK;

@@ -43,6 +43,24 @@ def test_fft_engine_matches_float64(mm, n, inverse):
     assert err < 2e-6, err
 
 
+@pytest.mark.parametrize("n", [478, 678])
+@pytest.mark.parametrize("lines", [1, 15, 16, 17, 340, 4881])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_prime_factor_lengths_at_line_group_edges(mm, n, lines, inverse):
+    """Lines around a group's 16, a plane of a tile and more groups than CTAs:
+    a float32 transform of n <= 678 points, fewer than 60 roundings of 6e-8 on
+    a value's way and each below the largest output."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n + lines)
+    x = torch.randn((n, lines, 2), generator=g, device="cuda")
+    want = torch.view_as_complex(x.double())
+    want = torch.fft.ifft(want, dim=0) * n if inverse else torch.fft.fft(want, dim=0)
+    L = mm["lib"].lib()
+    mm["lib"].check(L.mm_fft_c2c(mm["lib"].ptr(x), n, lines, int(inverse), mm["lib"].stream_ptr()))
+    err = (torch.view_as_complex(x).to(torch.complex128) - want).abs().max() / want.abs().max()
+    assert err < 60 * 6e-8, float(err)
+
+
 def _maxima_case(mm, im, raw, th, delta, dfit, sz=1.0, sxy=1.5):
     got = mm["maxima"].find_local_maxima(torch.from_numpy(im).cuda(), th, delta, dfit,
                                          torch.from_numpy(raw).cuda(), sz, sxy).cpu().numpy()

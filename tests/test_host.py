@@ -251,6 +251,53 @@ def test_rader_split_matches_the_dft(R, N1, N2, g, inverse):
     assert np.abs(X - want).max() <= 1e-12 * np.abs(want).max()
 
 
+@pytest.mark.parametrize("R,C,N1,N2,g", [(113, 6, 16, 7, 3), (239, 2, 14, 17, 7)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_prime_factor_tables_match_the_dft(R, C, N1, N2, g, inverse):
+    """The three phases of csrc/fft_pfa.cuh with the tables of pfa_tables
+    (csrc/fft_plan.cu), restated in NumPy for one line: every input and every
+    output place is used once and lies in the line."""
+    N, M = C * R, R - 1
+    gp = [pow(g, q, R) for q in range(M)]
+    q_of = {(q % N1, q % N2): q for q in range(M)}
+
+    def crt(a, b):
+        return next(k for k in range(b, N + 1, R) if k % C == a)
+
+    src = np.array([[[(R * c + C * gp[-q_of[q1, q2] % M]) % N for q2 in range(N2)] for c in range(C)]
+                    for q1 in range(N1)])
+    dst = np.array([[[crt(c, gp[q_of[q1, q2]]) for q2 in range(N2)] for c in range(C)] for q1 in range(N1)])
+    src0, dst0 = [R * c % N for c in range(C)], [crt(c, 0) for c in range(C)]
+    for places in (list(src.ravel()) + src0, list(dst.ravel()) + dst0):
+        assert sorted(places) == list(range(N))
+    h = np.zeros((N1, N2), complex)
+    for s in range(M):
+        h[s % N1, s % N2] = np.exp((2j if inverse else -2j) * np.pi * gp[s] / R) / M
+    H = np.fft.fft2(h)
+    rng = np.random.default_rng(N)
+    x = rng.standard_normal(N) + 1j * rng.standard_normal(N)
+    dft_c = (lambda v: np.fft.ifft(v, axis=0) * C) if inverse else (lambda v: np.fft.fft(v, axis=0))
+    x0 = dft_c(x[src0])
+    T = np.zeros((C, N1, N2), complex)
+    for q1 in range(N1):
+        T[:, q1] = np.fft.fft(dft_c(x[src[q1]]), axis=1)
+    y0 = np.zeros(C, complex)
+    for c in range(C):
+        for a2 in range(N2):
+            v = np.fft.fft(T[c, :, a2])
+            if a2 == 0:
+                y0[c] = x0[c] + v[0]
+            v = v * H[:, a2]
+            v[0] += x0[c] if a2 == 0 else 0
+            T[c, :, a2] = np.fft.ifft(v) * N1
+    X = np.zeros(N, complex)
+    for q1 in range(N1):
+        X[dst[q1]] = np.fft.ifft(T[:, q1], axis=1) * N2
+    X[dst0] = y0
+    want = np.fft.ifft(x) * N if inverse else np.fft.fft(x)
+    assert np.abs(X - want).max() <= 1e-12 * np.abs(want).max()
+
+
 def test_fov_graph_settings_follow_the_driver_defaults():
     """FovGraph reads a TOML section as hyb_spots does: None threshold -> NaN
     (every voxel), None blur -> -1 (no blur), delta > 5 -> TypeError."""
