@@ -158,6 +158,7 @@ struct Small {
     unsigned rows2;      // kept rows (set 2)
     unsigned overflow;   // largest candidate count that did not fit
     unsigned err;        // a kernel gave up a bounded wait (MM_ETIMEOUT)
+    unsigned queue[2];   // group counter of the persistent transform passes
     unsigned pad0_;
     double sumsq;
     float div;
@@ -303,6 +304,8 @@ int run_tiles(mm_ctx *c, TileGeom g, const void *image, int dtype, const float *
     if (!res && (rc = ws_get(c, WS_RES, sizeof(float) * tile_r * g.nt, &res, st))) return rc;
     if (rdelta >= 0 && (rc = ws_get(c, WS_TMP, sizeof(float) * tile_r * g.nt, &tmp, st))) return rc;
     float2 *S = (float2 *)spec;
+    Small *sm;
+    if ((rc = small_get(c, &sm, st))) return rc;
     const long long wstride = (long long)g.Zp * plane_c;
     // algorithmic bytes of each stage for this batch (its inputs read once, outputs written once)
     double in_b = 0;
@@ -317,26 +320,20 @@ int run_tiles(mm_ctx *c, TileGeom g, const void *image, int dtype, const float *
     }
     {
         StageTimer t(c, ST_COLS_FWD, 2 * spec_b, st);
-        if ((rc = mm_launch_cols(S, g.P, g.H, g.H, plane_c, g.nt * g.Z, false, st))) return rc;
+        if ((rc = mm_launch_cols(S, g.P, g.H, g.H, plane_c, g.nt * g.Z, false, sm->queue, st))) return rc;
     }
     const int zform = zform_of(c, g, zop);
     if (zform == MM_ZFORM_TENSOR) {
         // the matrix applied on the tensor cores; the z kernel is read once per batch
-        Small *sm;
-        if ((rc = small_get(c, &sm, st))) return rc;
         StageTimer t(c, ST_ZPASS, 2 * spec_b + 8.0 * wstride, st);
         if ((rc = mm_launch_zmma_apply(S, zop, g.Z, g.zpad, g.Zp, plane_c, g.nt, fresp, &sm->err, st))) return rc;
     } else if (zform == MM_ZFORM_REGISTERS && zth_takes(g, c->zform == MM_ZFORM_REGISTERS)) {
         // the matrix formed in registers, operands staged by TMA; the z kernel
         // is read once per batch
-        Small *sm;
-        if ((rc = small_get(c, &sm, st))) return rc;
         StageTimer t(c, ST_ZPASS, 2 * spec_b + 8.0 * wstride, st);
         if ((rc = mm_launch_zth_apply(S, zop, g.Z, g.zpad, g.Zp, plane_c, g.nt, fresp, &sm->err, st))) return rc;
     } else if (zform == MM_ZFORM_REGISTERS) {
         // the same with each tile's own z kernel, read once per tile
-        Small *sm;
-        if ((rc = small_get(c, &sm, st))) return rc;
         StageTimer t(c, ST_ZPASS, 2 * spec_b + (g.npsf == 1 ? 8.0 * wstride : w_b), st);
         if ((rc = mm_launch_zpt_apply(S, zop, wstride, g.Z, g.zpad, g.Zp, plane_c, g.t0, g.nt, g.npsf, fresp,
                                       &sm->err, st)))
@@ -357,7 +354,7 @@ int run_tiles(mm_ctx *c, TileGeom g, const void *image, int dtype, const float *
     }
     {
         StageTimer t(c, ST_COLS_INV, 2 * spec_b, st);
-        if ((rc = mm_launch_cols(S, g.P, g.H, g.H, plane_c, g.nt * g.Z, true, st))) return rc;
+        if ((rc = mm_launch_cols(S, g.P, g.H, g.H, plane_c, g.nt * g.Z, true, sm->queue, st))) return rc;
     }
     // with the blur folded and only the centre read, the stitched buffer is
     // written straight from the inverse pass
@@ -839,7 +836,7 @@ extern "C" int mm_tile_geometry(int Z, int X, int Y, int tile_size, int zpad, in
 
 extern "C" int mm_fft_c2c(void *data, int n, int nlines, int inverse, void *stream) {
     MM_REQUIRE(data && n >= 1 && nlines >= 1, "bad FFT arguments");
-    return mm_launch_cols((float2 *)data, n, nlines, nlines, 0, 1, inverse != 0, (cudaStream_t)stream);
+    return mm_launch_cols((float2 *)data, n, nlines, nlines, 0, 1, inverse != 0, nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int mm_profile_enable(mm_ctx *c, int on) {

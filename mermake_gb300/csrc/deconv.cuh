@@ -112,12 +112,14 @@ __device__ __host__ inline int mm_map_z(int j, int Z, int zpad, int Zp) {
     return mm_map_z0(q, Z, zpad);
 }
 
-// host launchers (deconv.cu)
+// host launchers (deconv.cu, fft_rows.cu, fft_cols.cu).  queue: two zero words
+// of the calling context's scratch, the group counter of the persistent
+// prime-factor passes (fft_pfa.cuh), or NULL
 int mm_launch_rows_fwd_img(const TileGeom &g, const void *img, int dtype, const float *flat, float2 *S,
                            cudaStream_t st);
 int mm_launch_rows_fwd_f32(const float *vol, int nrows, int P, float2 *S, cudaStream_t st);
 int mm_launch_cols(float2 *S, int n, long long se, int nlines, long long plane_stride, int nplanes,
-                   bool inv, cudaStream_t st);
+                   bool inv, unsigned *queue, cudaStream_t st);
 int mm_launch_zpass(const TileGeom &g, float2 *S, const float2 *W, long long wstride, cudaStream_t st);
 
 // z pass from the z kernel w (Zp, P, P/2+1) per spectrum, the inverse DFT of

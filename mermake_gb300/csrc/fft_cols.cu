@@ -52,14 +52,16 @@ k_cols(float2 *__restrict__ S, long long se, int nlines, long long plane_stride,
 template <int N, bool INV>
 __global__ void __launch_bounds__(PfaK<N>::threads, 2)
 k_cols_pfa(float2 *__restrict__ S, unsigned se8, int nlines, long long plane_stride, int total, int ngroups,
-           FftPlan P) {
+           FftPlan P, unsigned *__restrict__ queue) {
     using K = PfaK<N>;
-    extern __shared__ __align__(128) unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int next;
     const PfaSmem<N> s = pfa_layout<N>(smem_raw, sizeof(float2) * K::trows * kPfaNL);
     pfa_load_tables<N, INV>(s, P);
     __syncthreads();
     const int l = threadIdx.x % kPfaNL, q1 = threadIdx.x / kPfaNL;
-    for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
+    for (int grp = blockIdx.x; grp < ngroups;) {
+        const int asked = threadIdx.x == 0 ? queue_ask(queue, grp) : 0;
         // a line past the last one loads the last one and stores nothing
         const int line = min(grp * kPfaNL + l, total - 1);
         const bool mine = grp * kPfaNL + l < total;
@@ -90,7 +92,17 @@ k_cols_pfa(float2 *__restrict__ S, unsigned se8, int nlines, long long plane_str
         }
         __syncthreads();  // T is free: the previous group's last phase has read it
         pfa_put<N>(s, v, q1, l);
+        if (threadIdx.x == 0) next = asked;
         __syncthreads();
+        grp = next;
+        if (grp < ngroups) {
+            // the next group's 128-byte runs into L2, so that its loads wait
+            // for L2 only
+            const int n0 = grp * kPfaNL, pl = n0 / nlines;
+            const char *nb = reinterpret_cast<const char *>(S + pl * plane_stride + (n0 - pl * nlines));
+            for (int e = threadIdx.x; e < N; e += K::threads)
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(nb + (unsigned long long)(unsigned)e * se8));
+        }
         pfa_middle<N>(s, q1, l);
         __syncthreads();
         const int *op = s.tout + q1 * K::ipad;
@@ -107,32 +119,33 @@ k_cols_pfa(float2 *__restrict__ S, unsigned se8, int nlines, long long plane_str
             for (int c = 0; c < K::C; ++c) *at(s.out0[c]) = s.y0[c * kPfaNL + l];
         }
     }
+    if (threadIdx.x == 0) queue_leave(queue);
 }
 
 template <int N>
 int launch_pfa(float2 *S, unsigned se8, int nlines, long long plane_stride, int total, bool inv, const FftPlan &P,
-               cudaStream_t st) {
+               unsigned *queue, cudaStream_t st) {
     using K = PfaK<N>;
     const size_t sm = sizeof(float2) * K::trows * kPfaNL + pfa_tail_bytes<N>();
     int ngroups = mm_cdiv(total, kPfaNL);
     const void *fn = inv ? (const void *)k_cols_pfa<N, true> : (const void *)k_cols_pfa<N, false>;
     FftPlan Pa = P;
-    void *args[] = {&S, &se8, &nlines, &plane_stride, &total, &ngroups, &Pa};
+    void *args[] = {&S, &se8, &nlines, &plane_stride, &total, &ngroups, &Pa, &queue};
     return launch_fft_kernel(fn, dim3(fft_grid(ngroups, {K::threads, 2})), sm, st, args, K::threads);
 }
 
 }  // namespace
 
 int mm_launch_cols(float2 *S, int n, long long se, int nlines, long long plane_stride, int nplanes, bool inv,
-                   cudaStream_t st) {
+                   unsigned *queue, cudaStream_t st) {
     FftPlan P;
     int rc = mm_fft_plan_get(n, &P);
     if (rc) return rc;
     const long long total = (long long)nlines * nplanes;
     // element strides below 4 GB and a line count the kernel's ints hold
     if (P.pfa_idx && se * 8 < (1LL << 32) && total < (1LL << 31) - kPfaNL) {
-        if (n == 678) return launch_pfa<678>(S, (unsigned)(se * 8), nlines, plane_stride, (int)total, inv, P, st);
-        return launch_pfa<478>(S, (unsigned)(se * 8), nlines, plane_stride, (int)total, inv, P, st);
+        if (n == 678) return launch_pfa<678>(S, (unsigned)(se * 8), nlines, plane_stride, (int)total, inv, P, queue, st);
+        return launch_pfa<478>(S, (unsigned)(se * 8), nlines, plane_stride, (int)total, inv, P, queue, st);
     }
     int nl = pick_nl(P, 16, kColsCfg);
     size_t sm = fft_smem(P, nl, kColsCfg);

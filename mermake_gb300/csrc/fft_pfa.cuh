@@ -352,3 +352,19 @@ __device__ __forceinline__ void pfa_last(const PfaSmem<N> &s, int k1, int q1, in
     for (int a = 0; a < K::N2; ++a) v[a] = t[a * kPfaNL];
     pdft<K::N2, true>(v);
 }
+
+// ---- dynamic group order --------------------------------------------------
+// The persistent CTAs take groups from a counter: SMs finish a group at
+// different speeds (on 8 tiles of 678 the static order left the SMs active
+// 85 % of the pass on average, the slowest all of it).  queue: two words of
+// the context's scratch, zero between launches (the last CTA resets them);
+// NULL: every gridDim.x-th group.  Thread 0 asks at a group's start and
+// publishes the answer before a later barrier of the group.
+__device__ __forceinline__ int queue_ask(unsigned *queue, int grp) {
+    return queue ? (int)(gridDim.x + atomicAdd(queue, 1u)) : grp + (int)gridDim.x;
+}
+__device__ __forceinline__ void queue_leave(unsigned *queue) {
+    if (!queue) return;
+    __threadfence();
+    if (atomicAdd(queue + 1, 1u) == gridDim.x - 1) queue[0] = queue[1] = 0;
+}

@@ -99,7 +99,7 @@ int mm_wiener_build_impl(const float *psf, int pz, int px, int py, int tile_heig
     int rc;
     if ((rc = mm_launch_sum_parts(parts, 608, dsum, st))) return rc;
     if ((rc = mm_launch_rows_fwd_f32(vol, g.nz * g.nx, g.ny, S, st))) return rc;
-    if ((rc = mm_launch_cols(S, g.nx, H, H, (long long)g.nx * H, g.nz, false, st))) return rc;
+    if ((rc = mm_launch_cols(S, g.nx, H, H, (long long)g.nx * H, g.nz, false, nullptr, st))) return rc;
     if ((rc = mm_launch_zfwd(S, g.nz, g.nx * H, st))) return rc;
     k_wiener<<<608, 256, 0, st>>>(S, g.nz, g.nx, H, g.ny, beta, dsum, W);
     MM_CHECK_LAUNCH();
