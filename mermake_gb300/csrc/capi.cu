@@ -316,7 +316,7 @@ int run_tiles(mm_ctx *c, TileGeom g, const void *image, int dtype, const float *
     const double spec_b = 8.0 * tile_c * g.nt, real_b = 4.0 * tile_r * g.nt, w_b = 8.0 * wstride * g.nt;
     {
         StageTimer t(c, ST_ROWS_FWD, in_b + spec_b, st);
-        if ((rc = mm_launch_rows_fwd_img(g, image, dtype, flat, S, st))) return rc;
+        if ((rc = mm_launch_rows_fwd_img(g, image, dtype, flat, S, sm->queue, st))) return rc;
     }
     {
         StageTimer t(c, ST_COLS_FWD, 2 * spec_b, st);
@@ -361,11 +361,12 @@ int run_tiles(mm_ctx *c, TileGeom g, const void *image, int dtype, const float *
     const bool direct_stitch = fresp && win == -1 && !res_out && stitch;
     if (fresp && win >= -1 && !res_out) {
         StageTimer t(c, ST_ROWS_INV, spec_b + real_b, st);
-        if ((rc = mm_launch_rows_inv_win(S, g, win, (float *)res, direct_stitch ? stitch : nullptr, osz, osx, st)))
+        if ((rc = mm_launch_rows_inv_win(S, g, win, (float *)res, direct_stitch ? stitch : nullptr, osz, osx,
+                                         sm->queue, st)))
             return rc;
     } else {
         StageTimer t(c, ST_ROWS_INV, spec_b + real_b * (rdelta >= 0 ? 2 : 1), st);
-        if ((rc = mm_launch_rows_inv(S, g.nt * g.Z * g.P, g.P, g.H, (float *)res, (float *)tmp, rdelta, st)))
+        if ((rc = mm_launch_rows_inv(S, g.nt * g.Z * g.P, g.P, g.H, (float *)res, (float *)tmp, rdelta, sm->queue, st)))
             return rc;
     }
     if (rdelta >= 0 || (stitch && !direct_stitch)) {

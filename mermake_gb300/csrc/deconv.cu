@@ -41,12 +41,11 @@ int set_smem(K *kernel, size_t bytes) {
 // the flat), so the gathers do not stall on global latency row by row.
 // float32 tiles gather straight from global memory.
 // ---------------------------------------------------------------------------
-template <typename T, int LMAX, int NF, int NLF>
+template <typename T, int LMAX>
 __device__ __forceinline__ void rows_fwd_group(const TileGeom &g, const T *__restrict__ img,
                                                const float *__restrict__ flat, float2 *__restrict__ S,
                                                const FftPlan &P, int nl, const FftSmem &L, int bx, int by) {
-    if constexpr (NF > 0) nl = NLF;
-    const int n = NF > 0 ? NF : P.n;
+    const int n = P.n;
     const int ti = g.t0 + by;
     const TileDesc d = mm_tile_desc(g, ti);
     const long long nrows = (long long)g.Z * g.P;
@@ -59,7 +58,7 @@ __device__ __forceinline__ void rows_fwd_group(const TileGeom &g, const T *__res
         bool zero = true;
         for (int xp = (int)(row0 / g.Z); xp <= (int)(rl / g.Z); ++xp) zero &= mm_map_xy(xp, d.x == 0, d.xd, g.P, g.ov) < 0;
         if (zero) {
-            const int H = NF > 0 ? NF / 2 + 1 : g.H;
+            const int H = g.H;
             float2 *Sb = S + (long long)by * nrows * H;
             const int nr = (int)(rl - row0 + 1);
             for (int it = threadIdx.x; it < nr * H; it += blockDim.x) {
@@ -178,11 +177,11 @@ __device__ __forceinline__ void rows_fwd_group(const TileGeom &g, const T *__res
         }
     }
     __syncthreads();
-    float2 *R = fft_run<false, LMAX, NF, NLF>(L.A, L.B, nl, P, L.tw, L.tab, L.scr);
+    float2 *R = fft_lines<false, LMAX>(L.A, L.B, nl, P, L.tw, L.tab, L.scr);
 
     // unpack the two real rows of each line into their spectrum rows z P + x;
     // the spectrum row of each of the 2 nl rows goes in the (now idle) y map
-    const int H = NF > 0 ? NF / 2 + 1 : g.H;
+    const int H = g.H;
     const float invH = 1.0f / (float)H;
     float2 *Sb = S + (long long)by * nrows * H;
     int *drow = ymap;
@@ -202,9 +201,8 @@ __device__ __forceinline__ void rows_fwd_group(const TileGeom &g, const T *__res
     }
 }
 
-// persistent: the CTAs walk the groups (tables loaded once); NF > 0: the
-// engine specialised for length NF at NLF lines per CTA
-template <typename T, int LMAX, int NF = 0, int NLF = 0>
+// persistent: the CTAs walk the groups (tables loaded once)
+template <typename T, int LMAX>
 __global__ void __launch_bounds__(kRowsFwdCfg.threads, kRowsFwdCfg.ctas)
 k_rows_fwd_img(TileGeom g, const T *__restrict__ img, const float *__restrict__ flat,
                float2 *__restrict__ S, FftPlan P, int nl, int gx, int ngroups) {
@@ -213,7 +211,7 @@ k_rows_fwd_img(TileGeom g, const T *__restrict__ img, const float *__restrict__ 
     fft_load_tables(P, L.tw, L.tab);
     for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
         const int by = grp / gx;
-        rows_fwd_group<T, LMAX, NF, NLF>(g, img, flat, S, P, nl, L, grp - by * gx, by);
+        rows_fwd_group<T, LMAX>(g, img, flat, S, P, nl, L, grp - by * gx, by);
         __syncthreads();
     }
 }
@@ -267,7 +265,7 @@ struct StitchMap {
     const TileGeom *g;
 };
 
-template <int LMAX, int NF, int NLF>
+template <int LMAX>
 __device__ __forceinline__ void rows_inv_group(const float2 *__restrict__ S, long long nrows, int H,
                                                float *__restrict__ out, float *__restrict__ blur, int delta,
                                                const FftPlan &P, int nl, const FftSmem &L, long long row0,
@@ -275,11 +273,7 @@ __device__ __forceinline__ void rows_inv_group(const float2 *__restrict__ S, lon
     // rows [row0, nrows) of the group exist (nrows: the end of the group's
     // window, or of the batch); only columns [ylo, yhi) are stored, into `out`
     // (row-major, n per row) or the stitched FOV buffer (smap)
-    if constexpr (NF > 0) {
-        nl = NLF;
-        H = NF / 2 + 1;
-    }
-    const int n = NF > 0 ? NF : P.n;
+    const int n = P.n;
     const bool even = (n % 2) == 0;
     const float invH = 1.0f / (float)H, invn = 1.0f / (float)n;
     constexpr int U = 4;
@@ -310,7 +304,7 @@ __device__ __forceinline__ void rows_inv_group(const float2 *__restrict__ S, lon
         }
     }
     __syncthreads();
-    float2 *R = fft_run<true, LMAX, NF, NLF>(L.A, L.B, nl, P, L.tw, L.tab, L.scr);
+    float2 *R = fft_lines<true, LMAX>(L.A, L.B, nl, P, L.tw, L.tab, L.scr);
     const float *Rf = reinterpret_cast<const float *>(R);
     for (int it = threadIdx.x; it < 2 * nl * n; it += blockDim.x) {
         const int q = fdiv_i(it, n, invn), e = it - q * n;
@@ -368,9 +362,8 @@ __device__ __forceinline__ void rows_inv_group(const float2 *__restrict__ S, lon
     }
 }
 
-// persistent: the CTAs walk the row groups (tables loaded once); NF > 0 as
-// for k_rows_fwd_img
-template <int LMAX, int NF = 0, int NLF = 0>
+// persistent: the CTAs walk the row groups (tables loaded once)
+template <int LMAX>
 __global__ void __launch_bounds__(kRowsInvCfg.threads, kRowsInvCfg.ctas)
 k_rows_inv(const float2 *__restrict__ S, long long nrows, int H, float *__restrict__ out,
            float *__restrict__ blur, int delta, FftPlan P, int nl, int ngroups) {
@@ -378,25 +371,9 @@ k_rows_inv(const float2 *__restrict__ S, long long nrows, int H, float *__restri
     const FftSmem L = fft_smem_layout(smem_raw, P, nl);
     fft_load_tables(P, L.tw, L.tab);
     for (int grp = blockIdx.x; grp < ngroups; grp += gridDim.x) {
-        rows_inv_group<LMAX, NF, NLF>(S, nrows, H, out, blur, delta, P, nl, L, (long long)grp * 2 * nl);
+        rows_inv_group<LMAX>(S, nrows, H, out, blur, delta, P, nl, L, (long long)grp * 2 * nl);
         __syncthreads();
     }
-}
-
-// The rows and columns of tile t (of the batch) that the caller reads: the
-// window [lo, hi) of padded indices along x and y, from the tile's yielded
-// extent.  reach >= 0: the hyb keep band, [ov - reach, extent - ov + reach);
-// reach < 0: the stitched centre, [ov, extent - ov).
-__device__ __forceinline__ void read_window(const TileGeom &g, int t, int reach, int &xlo, int &xhi, int &ylo,
-                                            int &yhi) {
-    const TileDesc d = mm_tile_desc(g, g.t0 + t);
-    const int r = reach < 0 ? 0 : reach;
-    xlo = max(0, g.ov - r);
-    ylo = max(0, g.ov - r);
-    xhi = min(d.xend, d.xend - g.ov + r);
-    yhi = min(d.yend, d.yend - g.ov + r);
-    if (xhi < xlo) xhi = xlo;
-    if (yhi < ylo) yhi = ylo;
 }
 
 // The inverse y pass over the read windows only: per tile, the rows x in
@@ -405,7 +382,7 @@ __device__ __forceinline__ void read_window(const TileGeom &g, int t, int reach,
 // outside are not written.  The CTAs first tabulate the groups per tile
 // (tiles <= kMaxWinTiles), then walk the groups as k_rows_inv does.
 constexpr int kMaxWinTiles = 256;
-template <int LMAX, int NF = 0, int NLF = 0>
+template <int LMAX>
 __global__ void __launch_bounds__(kRowsInvCfg.threads, kRowsInvCfg.ctas)
 k_rows_inv_win(const float2 *__restrict__ S, TileGeom g, int reach, float *__restrict__ out, FftPlan P, int nl,
                int cum_off, float *__restrict__ stitch, long long osz, long long osx) {
@@ -413,7 +390,6 @@ k_rows_inv_win(const float2 *__restrict__ S, TileGeom g, int reach, float *__res
     int *cum = reinterpret_cast<int *>(smem_raw + cum_off);  // groups before tile t (nt + 1 entries)
     const FftSmem L = fft_smem_layout(smem_raw, P, nl);
     fft_load_tables(P, L.tw, L.tab);
-    if constexpr (NF > 0) nl = NLF;
     const int gr = 2 * nl;
     if (threadIdx.x == 0) {
         int acc = 0;
@@ -448,9 +424,9 @@ k_rows_inv_win(const float2 *__restrict__ S, TileGeom g, int reach, float *__res
             sm.base = base; sm.z = z; sm.ti = g.t0 + t; sm.xlo = xlo;
             sm.d = mm_tile_desc(g, g.t0 + t);
             sm.g = &g;
-            rows_inv_group<LMAX, NF, NLF>(S, base + xhi, g.H, out, nullptr, -1, P, nl, L, row0, ylo, yhi, &sm);
+            rows_inv_group<LMAX>(S, base + xhi, g.H, out, nullptr, -1, P, nl, L, row0, ylo, yhi, &sm);
         } else {
-            rows_inv_group<LMAX, NF, NLF>(S, base + xhi, g.H, out, nullptr, -1, P, nl, L, row0, ylo, yhi);
+            rows_inv_group<LMAX>(S, base + xhi, g.H, out, nullptr, -1, P, nl, L, row0, ylo, yhi);
         }
         __syncthreads();
     }
@@ -578,10 +554,11 @@ __global__ void k_make_raw(TileGeom g, const T *__restrict__ img, const float *_
 // host launchers
 // ---------------------------------------------------------------------------
 int mm_launch_rows_fwd_img(const TileGeom &g, const void *img, int dtype, const float *flat, float2 *S,
-                           cudaStream_t st) {
+                           unsigned *queue, cudaStream_t st) {
     FftPlan P;
     int rc = mm_fft_plan_get(g.P, &P);
     if (rc) return rc;
+    if (mm_rows_pfa_takes(P, (long long)g.nt * g.Z * g.P)) return mm_launch_rows_fwd_pfa(g, img, dtype, flat, S, P, queue, st);
     // lines per CTA, with room after the scratch for the y map (P ints), which
     // later holds the spectrum rows of the CTA's 2 nl <= 32 rows
     const size_t mapb = sizeof(int) * (size_t)(P.n > 32 ? P.n : 32);
@@ -595,8 +572,8 @@ int mm_launch_rows_fwd_img(const TileGeom &g, const void *img, int dtype, const 
     const void *imga = img;
     const float *fa = flat;
     void *args[] = {&ga, &imga, &fa, &S, &P, &nl, &gx, &ngroups};
-    const void *fn = dtype == MM_DTYPE_U16 ? MM_FFT_KERNEL(P, nl, 8, k_rows_fwd_img, uint16_t,)
-                                          : MM_FFT_KERNEL(P, nl, 8, k_rows_fwd_img, float,);
+    const void *fn = dtype == MM_DTYPE_U16 ? MM_BY_CLASS(P, k_rows_fwd_img, uint16_t,)
+                                          : MM_BY_CLASS(P, k_rows_fwd_img, float,);
     return launch_fft_kernel(fn, grid, sm, st, args, kRowsFwdCfg.threads);
 }
 
@@ -612,10 +589,12 @@ int mm_launch_rows_fwd_f32(const float *vol, int nrows, int Pn, float2 *S, cudaS
 }
 
 int mm_launch_rows_inv(const float2 *S, int nrows, int Pn, int H, float *out, float *blur, int delta,
-                       cudaStream_t st) {
+                       unsigned *queue, cudaStream_t st) {
     FftPlan P;
     int rc = mm_fft_plan_get(Pn, &P);
     if (rc) return rc;
+    if (mm_rows_pfa_takes(P, nrows) && mm_rows_inv_pfa_fits(P, delta))
+        return mm_launch_rows_inv_pfa(S, nrows, out, blur, delta, P, queue, st);
     // the y blur's reciprocal table goes in the scratch: room for 2 delta + 2 floats
     auto bytes = [&](int l) {
         const size_t scr = sizeof(float4) * fft_scr_f4(P, l, kRowsInvCfg.threads / 32);
@@ -630,17 +609,19 @@ int mm_launch_rows_inv(const float2 *S, int nrows, int Pn, int H, float *out, fl
     long long nr = nrows;
     int ngroups = mm_cdiv(nrows, 2 * nl);
     void *args[] = {&S, &nr, &H, &out, &blur, &delta, &P, &nl, &ngroups};
-    return launch_fft_kernel(MM_FFT_KERNEL(P, nl, 8, k_rows_inv, ), dim3(fft_grid(ngroups, kRowsInvCfg)), sm, st, args,
+    return launch_fft_kernel(MM_BY_CLASS(P, k_rows_inv, ), dim3(fft_grid(ngroups, kRowsInvCfg)), sm, st, args,
                              kRowsInvCfg.threads);
 }
 
 int mm_launch_rows_inv_win(const float2 *S, const TileGeom &g, int reach, float *out, float *stitch, long long osz,
-                           long long osx, cudaStream_t st) {
+                           long long osx, unsigned *queue, cudaStream_t st) {
     MM_REQUIRE(!stitch || reach < 0, "stitching stores the centre window only");
     FftPlan P;
     int rc = mm_fft_plan_get(g.P, &P);
     if (rc) return rc;
     MM_REQUIRE(g.nt <= kMaxWinTiles, "windowed inverse pass takes at most %d tiles per batch", kMaxWinTiles);
+    if (mm_rows_pfa_takes(P, (long long)g.nt * g.Z * g.P))
+        return mm_launch_rows_inv_win_pfa(S, g, reach, out, stitch, osz, osx, P, queue, st);
     const size_t lim = (size_t)fft_smem_limit(kRowsInvCfg);
     const size_t cumb = sizeof(int) * ((size_t)g.nt + 1);
     auto bytes = [&](int l) { return ((fft_smem(P, l, kRowsInvCfg) + 15) & ~(size_t)15) + cumb; };
@@ -653,7 +634,7 @@ int mm_launch_rows_inv_win(const float2 *S, const TileGeom &g, int reach, float 
     const long long ngroups = (long long)g.nt * g.Z * mm_cdiv(g.P, 2 * nl);
     TileGeom ga = g;
     void *args[] = {&S, &ga, &reach, &out, &P, &nl, &cum_off, &stitch, &osz, &osx};
-    return launch_fft_kernel(MM_FFT_KERNEL(P, nl, 8, k_rows_inv_win, ), dim3(fft_grid(ngroups, kRowsInvCfg)), sm, st,
+    return launch_fft_kernel(MM_BY_CLASS(P, k_rows_inv_win, ), dim3(fft_grid(ngroups, kRowsInvCfg)), sm, st,
                              args, kRowsInvCfg.threads);
 }
 

@@ -112,11 +112,38 @@ __device__ __host__ inline int mm_map_z(int j, int Z, int zpad, int Zp) {
     return mm_map_z0(q, Z, zpad);
 }
 
+#ifdef __CUDACC__
+// The rows and columns of tile t (of the batch) that the caller reads: the
+// window [lo, hi) of padded indices along x and y, from the tile's yielded
+// extent.  reach >= 0: the hyb keep band, [ov - reach, extent - ov + reach);
+// reach < 0: the stitched centre, [ov, extent - ov).
+__device__ __forceinline__ void read_window(const TileGeom &g, int t, int reach, int &xlo, int &xhi, int &ylo,
+                                            int &yhi) {
+    const TileDesc d = mm_tile_desc(g, g.t0 + t);
+    const int r = reach < 0 ? 0 : reach;
+    xlo = max(0, g.ov - r);
+    ylo = max(0, g.ov - r);
+    xhi = min(d.xend, d.xend - g.ov + r);
+    yhi = min(d.yend, d.yend - g.ov + r);
+    if (xhi < xlo) xhi = xlo;
+    if (yhi < ylo) yhi = ylo;
+}
+#endif
+
 // host launchers (deconv.cu, fft_rows.cu, fft_cols.cu).  queue: two zero words
 // of the calling context's scratch, the group counter of the persistent
 // prime-factor passes (fft_pfa.cuh), or NULL
 int mm_launch_rows_fwd_img(const TileGeom &g, const void *img, int dtype, const float *flat, float2 *S,
-                           cudaStream_t st);
+                           unsigned *queue, cudaStream_t st);
+// the y passes of the prime-factor lengths (fft_rows.cu)
+bool mm_rows_pfa_takes(const FftPlan &P, long long nrows);
+int mm_launch_rows_fwd_pfa(const TileGeom &g, const void *img, int dtype, const float *flat, float2 *S,
+                           const FftPlan &P, unsigned *queue, cudaStream_t st);
+bool mm_rows_inv_pfa_fits(const FftPlan &P, int delta);
+int mm_launch_rows_inv_pfa(const float2 *S, long long nrows, float *out, float *blur, int delta, const FftPlan &P,
+                           unsigned *queue, cudaStream_t st);
+int mm_launch_rows_inv_win_pfa(const float2 *S, const TileGeom &g, int reach, float *out, float *stitch, long long osz,
+                               long long osx, const FftPlan &P, unsigned *queue, cudaStream_t st);
 int mm_launch_rows_fwd_f32(const float *vol, int nrows, int P, float2 *S, cudaStream_t st);
 int mm_launch_cols(float2 *S, int n, long long se, int nlines, long long plane_stride, int nplanes,
                    bool inv, unsigned *queue, cudaStream_t st);
@@ -170,14 +197,14 @@ int mm_launch_zpt_apply(float2 *S, const float2 *w, long long wstride, int Z, in
 int mm_blur_response_get(int P, int delta, const float **out);
 int mm_launch_zfwd(float2 *S, int Zp, int plane, cudaStream_t st);
 int mm_launch_rows_inv(const float2 *S, int nrows, int P, int H, float *out, float *blur, int delta,
-                       cudaStream_t st);
+                       unsigned *queue, cudaStream_t st);
 // the inverse y pass (no blur) over the rows and columns of each tile that the
 // caller reads: reach >= 0, the band [ov - reach, extent - ov + reach) of the
 // hyb keep filter; reach < 0, the stitched centre [ov, extent - ov)
 // (reach < 0 with `stitch` given: the centre goes straight into the stitched
 // FOV buffer, strides osz, osx, in Deconvolver.apply's overwrite order)
 int mm_launch_rows_inv_win(const float2 *S, const TileGeom &g, int reach, float *out, float *stitch, long long osz,
-                           long long osx, cudaStream_t st);
+                           long long osx, unsigned *queue, cudaStream_t st);
 int mm_launch_blur_x_sub(const TileGeom &g, const float *res, const float *tmp, int delta,
                          float *res_out, float *stitch, long long osz, long long osx, cudaStream_t st);
 int mm_launch_make_raw(const TileGeom &g, const void *img, int dtype, const float *flat, float *raw,
