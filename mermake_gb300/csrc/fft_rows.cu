@@ -82,92 +82,84 @@ __device__ __forceinline__ void pfa_take(const PfaSmem<N> &s, float2 (&v)[PfaK<N
 // takes half sums); the y padding is in the input table, which holds the place
 // of the pixel that each padded column copies, or the row of zeros.
 // ---------------------------------------------------------------------------
+// All of a line's loads are issued before the first is used (U words or pixels
+// per lane cover the longest row), so a line waits for memory once.
 __device__ __forceinline__ float half_over(const float *f) { return f ? __fdividef(0.5f, *f) : 0.5f; }
 
+template <int N>
 __device__ __forceinline__ void stage_rows(const uint16_t *ra, const uint16_t *rb, const float *fr, int n,
                                            float2 *dst, int lane) {
-    if (!rb || ((reinterpret_cast<uintptr_t>(ra) ^ reinterpret_cast<uintptr_t>(rb)) & 2)) {
-        // one row, or two rows of different alignment: pixel by pixel
-        for (int y0 = lane; y0 < n; y0 += 32 * 4) {
-            float a[4], b[4], f[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int y = y0 + 32 * u;
-                a[u] = b[u] = f[u] = 0.f;
-                if (y < n) {
-                    a[u] = (float)ra[y];
-                    if (rb) b[u] = (float)rb[y];
-                    f[u] = half_over(fr ? fr + y : nullptr);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (y0 + 32 * u < n) dst[(y0 + 32 * u) * kPitch] = pmul(make_float2(a[u], b[u]), f[u]);
-        }
-        return;
-    }
-    // words of two pixels, y = 2 w - off and the next; the words that reach
-    // past either end of the row are read as their one pixel
+    // words of two pixels of row a, y = 2 w - off and the next; the words that
+    // reach past either end of the row are read as their one pixel.  Row b
+    // comes the same way, or pixel by pixel where it starts on the other half
+    // of a word.
+    constexpr int U = (N / 2 + 1 + 31) / 32;
     const int off = (int)((reinterpret_cast<uintptr_t>(ra) >> 1) & 1);
     const unsigned *wa = reinterpret_cast<const unsigned *>(ra - off);
+    const bool same = rb && !((reinterpret_cast<uintptr_t>(ra) ^ reinterpret_cast<uintptr_t>(rb)) & 2);
     const unsigned *wb = reinterpret_cast<const unsigned *>(rb - off);
-    const int nw = (n + off + 1) / 2;
-    constexpr int U = 4;
-    for (int w0 = lane; w0 < nw; w0 += 32 * U) {
-        unsigned a[U], b[U];
-        float f0[U], f1[U];
+    unsigned a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int w = lane + 32 * u, y = 2 * w - off;
+        const bool lo = y >= 0 && y < n, hi = y + 1 < n;
+        a[u] = lo && hi ? wa[w] : lo ? ra[y] : hi ? (unsigned)ra[y + 1] << 16 : 0u;
+    }
+    if (same) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int w = w0 + 32 * u, y = 2 * w - off;
-            a[u] = b[u] = 0;
-            f0[u] = f1[u] = 0.f;
-            const bool lo = w < nw && y >= 0, hi = w < nw && y + 1 < n;
-            if (lo && hi) {
-                a[u] = wa[w];
-                b[u] = wb[w];
-            } else if (lo) {
-                a[u] = ra[y];
-                b[u] = rb[y];
-            } else if (hi) {
-                a[u] = (unsigned)ra[y + 1] << 16;
-                b[u] = (unsigned)rb[y + 1] << 16;
-            }
-            if (lo) f0[u] = half_over(fr ? fr + y : nullptr);
-            if (hi) f1[u] = half_over(fr ? fr + y + 1 : nullptr);
+            const int w = lane + 32 * u, y = 2 * w - off;
+            const bool lo = y >= 0 && y < n, hi = y + 1 < n;
+            b[u] = lo && hi ? wb[w] : lo ? rb[y] : hi ? (unsigned)rb[y + 1] << 16 : 0u;
         }
+    } else {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int w = w0 + 32 * u, y = 2 * w - off;
-            // 0x4B00xxxx is 2^23 + xxxx: the pixel as a float, exactly
-            const float2 m = make_float2(8388608.f, 8388608.f);
-            const float2 v0 = psub(make_float2(__uint_as_float(__byte_perm(a[u], 0x4B000000u, 0x7610)),
-                                               __uint_as_float(__byte_perm(b[u], 0x4B000000u, 0x7610))), m);
-            const float2 v1 = psub(make_float2(__uint_as_float(__byte_perm(a[u], 0x4B000000u, 0x7632)),
-                                               __uint_as_float(__byte_perm(b[u], 0x4B000000u, 0x7632))), m);
-            if (w < nw && y >= 0) dst[y * kPitch] = pmul(v0, f0[u]);
-            if (w < nw && y + 1 < n) dst[(y + 1) * kPitch] = pmul(v1, f1[u]);
+            const int y = 2 * (lane + 32 * u) - off;
+            const unsigned lo = rb && y >= 0 && y < n ? rb[y] : 0u, hi = rb && y + 1 < n ? rb[y + 1] : 0u;
+            b[u] = lo | hi << 16;
         }
+    }
+    // the two pixels of a word go out in the order that spreads a half warp's
+    // 16 stores over all banks: lanes 8 .. 15 of each half start with the second
+    const bool swap = lane & 8;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int y = 2 * (lane + 32 * u) - off;
+        // 0x4B00xxxx is 2^23 + xxxx: the pixel as a float, exactly
+        const unsigned p0 = swap ? 0x7632 : 0x7610, p1 = swap ? 0x7610 : 0x7632;
+        const int y0 = y + (swap ? 1 : 0), y1 = y + (swap ? 0 : 1);
+        const float2 m = make_float2(8388608.f, 8388608.f);
+        const float2 v0 = psub(make_float2(__uint_as_float(__byte_perm(a[u], 0x4B000000u, p0)),
+                                           __uint_as_float(__byte_perm(b[u], 0x4B000000u, p0))), m);
+        const float2 v1 = psub(make_float2(__uint_as_float(__byte_perm(a[u], 0x4B000000u, p1)),
+                                           __uint_as_float(__byte_perm(b[u], 0x4B000000u, p1))), m);
+        if (y0 >= 0 && y0 < n) dst[y0 * kPitch] = pmul(v0, half_over(fr ? fr + y0 : nullptr));
+        if (y1 >= 0 && y1 < n) dst[y1 * kPitch] = pmul(v1, half_over(fr ? fr + y1 : nullptr));
     }
 }
+template <int N>
 __device__ __forceinline__ void stage_rows(const float *ra, const float *rb, const float *fr, int n, float2 *dst,
                                            int lane) {
-    constexpr int U = 4;
-    for (int y0 = lane; y0 < n; y0 += 32 * U) {
-        float a[U], b[U], f[U];
+    constexpr int U = (N + 31) / 32;
+    float a[U], b[U];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int y = y0 + 32 * u;
-            a[u] = b[u] = f[u] = 0.f;
-            if (y < n) {
-                a[u] = ra[y];
-                if (rb) b[u] = rb[y];
-                f[u] = half_over(fr ? fr + y : nullptr);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-            if (y0 + 32 * u < n) dst[(y0 + 32 * u) * kPitch] = pmul(make_float2(a[u], b[u]), f[u]);
+    for (int u = 0; u < U; ++u) {
+        const int y = lane + 32 * u;
+        a[u] = y < n ? ra[y] : 0.f;
+        b[u] = rb && y < n ? rb[y] : 0.f;
     }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int y = lane + 32 * u;
+        if (y < n) dst[y * kPitch] = pmul(make_float2(a[u], b[u]), half_over(fr ? fr + y : nullptr));
+    }
+}
+
+// rows of `bytes` bytes at p into L2, a lane per 128 bytes
+__device__ __forceinline__ void prefetch_row(const void *p, int bytes, int lane) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)127, e = reinterpret_cast<uintptr_t>(p) + bytes;
+    for (uintptr_t c = a + 128 * lane; c < e; c += 128 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(c));
 }
 
 template <typename T, int N>
@@ -240,16 +232,29 @@ k_rows_fwd_pfa(TileGeom g, const T *__restrict__ img, const float *__restrict__ 
                 }
             }
             if (ra)
-                stage_rows(ra, rb, fr, d.yd, dst, lane);
+                stage_rows<N>(ra, rb, fr, d.yd, dst, lane);
             else
                 for (int y = lane; y < d.yd; y += 32) dst[y * kPitch] = make_float2(0.f, 0.f);
         }
+        if (tid == 0) next = asked;
         __syncthreads();
+        grp = next;
+        if (grp < ngroups && grp / gx == by) {
+            // the next group's pixel rows into L2 (past the rows of this one:
+            // a group is 16 lines of the same or the next x)
+            const int N0 = (grp - by * gx) * kPfaNL;
+            for (int q = warp; q < kPfaNL && N0 + q < LT; q += nw) {
+                const int x = (N0 + q) / zp, k = N0 + q - x * zp;
+                const int sx = mm_map_xy(x, d.x == 0, d.xd, N, g.ov);
+                if (sx < 0) continue;
+                const T *ra = img + 2 * k * g.isz + (long long)(d.x0 + sx) * g.isx + d.y0;
+                prefetch_row(ra, d.yd * (int)sizeof(T), lane);
+                if (2 * k + 1 < g.Z) prefetch_row(ra + g.isz, d.yd * (int)sizeof(T), lane);
+            }
+        }
         float2 v[K::C][K::N2], x0[K::C];
         pfa_take<N>(s, v, x0, q1, l);
-        if (tid == 0) next = asked;
         pfa_lines<N, false>(s, v, x0, q1, l);
-        grp = next;
         __syncthreads();
         // the two real rows' half spectra of each line
         for (int q = warp; q < kPfaNL; q += nw) {
@@ -369,12 +374,22 @@ k_rows_inv_pfa(const float2 *__restrict__ S, long long nrows, TileGeom g, int re
                 }
             }
         }
+        if (tid == 0) next = asked;
         __syncthreads();
+        grp = next;
+        if (!WIN || grp < cum[t + 1]) {
+            // the next group's spectrum rows into L2
+            const int N0 = WIN ? (grp - cum[t]) * kPfaNL : grp * kPfaNL;
+            const long long end = WIN ? (long long)g.Z * np : nrows / 2;
+            for (int q = warp; q < kPfaNL && N0 + q < end; q += nw) {
+                const int z = WIN ? (N0 + q) / np : 0;
+                const long long row = WIN ? tbase + (long long)z * N + (xlo & ~1) + 2 * (N0 + q - z * np) : 2LL * (N0 + q);
+                prefetch_row(S + row * H, 2 * H * 8, lane);
+            }
+        }
         float2 v[K::C][K::N2], x0[K::C];
         pfa_take<N>(s, v, x0, q1, l);
-        if (tid == 0) next = asked;
         pfa_lines<N, true>(s, v, x0, q1, l);
-        grp = next;
         __syncthreads();
         for (int q = warp; q < nl; q += nw) {
             int z, x;
@@ -409,26 +424,26 @@ k_rows_inv_pfa(const float2 *__restrict__ S, long long nrows, TileGeom g, int re
             if (WIN || delta < 0) continue;
             // y box mean of both rows: each lane slides a window along a
             // segment (an odd number of elements: lanes in distinct banks),
-            // the means replace the line in A once every lane has them
+            // and the sums wait in registers until every lane is through
             constexpr int seg = ((N + 31) / 32) | 1;
             const int s0 = lane * seg;
-            float2 m[seg];
-            if (s0 < N) {
-                float2 sum = make_float2(0.f, 0.f);
+            float2 m[seg], sum = make_float2(0.f, 0.f);
+            if (s0 < N)
                 for (int i = max(s0 - delta, 0); i <= min(s0 + delta, N - 1); ++i) sum = padd(sum, A[i * kPitch + q]);
+            const float2 *pa = A + (s0 + delta) * kPitch + q, *pd = A + (s0 - delta - 1) * kPitch + q;
 #pragma unroll
-                for (int u = 0; u < seg; ++u) {
-                    const int e = s0 + u, add = e + delta, drop = e - delta - 1;
-                    if (u > 0 && add <= N - 1) sum = padd(sum, A[add * kPitch + q]);
-                    if (u > 0 && drop >= 0 && e < N) sum = psub(sum, A[drop * kPitch + q]);
-                    // past the row's end: any count, not stored
-                    m[u] = pmul(sum, rtab[max(min(add, N - 1) - max(e - delta, 0) + 1, 0)]);
-                }
+            for (int u = 0; u < seg; ++u) {
+                const int e = s0 + u;
+                if (u > 0 && e + delta < N) sum = padd(sum, pa[u * kPitch]);
+                if (u > 0 && e > delta && e < N) sum = psub(sum, pd[u * kPitch]);
+                m[u] = sum;
             }
             __syncwarp();
 #pragma unroll
-            for (int u = 0; u < seg; ++u)
-                if (s0 + u < N) A[(s0 + u) * kPitch + q] = m[u];
+            for (int u = 0; u < seg; ++u) {
+                const int e = s0 + u;
+                if (e < N) A[e * kPitch + q] = pmul(m[u], rtab[min(e + delta, N - 1) - max(e - delta, 0) + 1]);
+            }
             __syncwarp();
             float *b0 = blur + r0 * N, *b1 = b0 + N;
 #pragma unroll 4
