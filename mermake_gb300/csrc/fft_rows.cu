@@ -43,11 +43,16 @@ __device__ __forceinline__ void pfa_lines(const PfaSmem<N> &s, float2 (&v)[PfaK<
     for (int c = 0; c < K::C; ++c) pfa_last<N>(s, c, q1, l, v[c]);
     __syncthreads();  // T has been read: A again
     unsigned char *A = reinterpret_cast<unsigned char *>(s.T) + l * 8;
-    const int *op = s.tout + q1 * K::ipad;
+    const int4 *op = reinterpret_cast<const int4 *>(s.tout + q1 * K::ipad);
 #pragma unroll
-    for (int c = 0; c < K::C; ++c)
+    for (int c = 0; c < K::ipad / 4; ++c) {
+        const int4 i4 = op[c];
+        const int e[4] = {i4.x, i4.y, i4.z, i4.w};
 #pragma unroll
-        for (int q = 0; q < K::N2; ++q) *reinterpret_cast<float2 *>(A + op[c * K::N2 + q]) = v[c][q];
+        for (int u = 0; u < 4; ++u)
+            if (4 * c + u < K::vals)
+                *reinterpret_cast<float2 *>(A + e[u]) = v[(4 * c + u) / K::N2][(4 * c + u) % K::N2];
+    }
     if (q1 == 0) {
 #pragma unroll
         for (int c = 0; c < K::C; ++c) *reinterpret_cast<float2 *>(A + s.out0[c]) = s.y0[c * kPfaNL + l];
@@ -83,76 +88,110 @@ __device__ __forceinline__ void pfa_take(const PfaSmem<N> &s, float2 (&v)[PfaK<N
 // of the pixel that each padded column copies, or the row of zeros.
 // ---------------------------------------------------------------------------
 // All of a line's loads are issued before the first is used (U words or pixels
-// per lane cover the longest row), so a line waits for memory once.
-__device__ __forceinline__ float half_over(const float *f) { return f ? __fdividef(0.5f, *f) : 0.5f; }
+// per lane cover the longest row), so a line waits for memory once, and the
+// addresses are a lane's base plus constants.
+__device__ __forceinline__ float half_over(float f) { return __fdividef(0.5f, f); }
 
+// 0x4B00xxxx is 2^23 + xxxx: the half word `sel` of a and b as floats, exactly
+__device__ __forceinline__ float2 two_pixels(unsigned a, unsigned b, unsigned sel) {
+    return psub(make_float2(__uint_as_float(__byte_perm(a, 0x4B000000u, sel)),
+                            __uint_as_float(__byte_perm(b, 0x4B000000u, sel))),
+                make_float2(8388608.f, 8388608.f));
+}
 template <int N>
-__device__ __forceinline__ void stage_rows(const uint16_t *ra, const uint16_t *rb, const float *fr, int n,
-                                           float2 *dst, int lane) {
-    // words of two pixels of row a, y = 2 w - off and the next; the words that
-    // reach past either end of the row are read as their one pixel.  Row b
-    // comes the same way, or pixel by pixel where it starts on the other half
-    // of a word.
+__device__ __forceinline__ void stage_rows(const uint16_t *ra, const uint16_t *rb, const float *fr, const float *hf,
+                                           int n, float2 *dst, int lane) {
+    // words of two pixels of row a, y = 2 w - off and the next, for the words
+    // inside the row; row b the same way, or pixel by pixel where it starts on
+    // the other half of a word
     constexpr int U = (N / 2 + 1 + 31) / 32;
     const int off = (int)((reinterpret_cast<uintptr_t>(ra) >> 1) & 1);
-    const unsigned *wa = reinterpret_cast<const unsigned *>(ra - off);
-    const bool same = rb && !((reinterpret_cast<uintptr_t>(ra) ^ reinterpret_cast<uintptr_t>(rb)) & 2);
-    const unsigned *wb = reinterpret_cast<const unsigned *>(rb - off);
+    const unsigned *wa = reinterpret_cast<const unsigned *>(ra - off) + lane;
+    const int y = 2 * lane - off;
+    const unsigned first = lane - off, count = (n + off) / 2 - off;  // word u is inside: first + 32 u < count
     unsigned a[U], b[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int w = lane + 32 * u, y = 2 * w - off;
-        const bool lo = y >= 0 && y < n, hi = y + 1 < n;
-        a[u] = lo && hi ? wa[w] : lo ? ra[y] : hi ? (unsigned)ra[y + 1] << 16 : 0u;
-    }
-    if (same) {
+    for (int u = 0; u < U; ++u) a[u] = first + 32 * u < count ? wa[32 * u] : 0u;
+    if (!rb) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int w = lane + 32 * u, y = 2 * w - off;
-            const bool lo = y >= 0 && y < n, hi = y + 1 < n;
-            b[u] = lo && hi ? wb[w] : lo ? rb[y] : hi ? (unsigned)rb[y + 1] << 16 : 0u;
-        }
+        for (int u = 0; u < U; ++u) b[u] = 0u;
+    } else if (!((reinterpret_cast<uintptr_t>(ra) ^ reinterpret_cast<uintptr_t>(rb)) & 2)) {
+        const unsigned *wb = reinterpret_cast<const unsigned *>(rb - off) + lane;
+#pragma unroll
+        for (int u = 0; u < U; ++u) b[u] = first + 32 * u < count ? wb[32 * u] : 0u;
     } else {
+        const uint16_t *pb = rb + y;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int y = 2 * (lane + 32 * u) - off;
-            const unsigned lo = rb && y >= 0 && y < n ? rb[y] : 0u, hi = rb && y + 1 < n ? rb[y + 1] : 0u;
-            b[u] = lo | hi << 16;
-        }
+        for (int u = 0; u < U; ++u)
+            b[u] = first + 32 * u < count ? pb[64 * u] | (unsigned)pb[64 * u + 1] << 16 : 0u;
     }
     // the two pixels of a word go out in the order that spreads a half warp's
     // 16 stores over all banks: lanes 8 .. 15 of each half start with the second
-    const bool swap = lane & 8;
+    const int sw = (lane >> 3) & 1;
+    const unsigned p0 = sw ? 0x7632 : 0x7610, p1 = sw ? 0x7610 : 0x7632;
+    float2 *d0 = dst + (y + sw) * kPitch, *d1 = dst + (y + 1 - sw) * kPitch;
+    if (hf) {
+        const float *f0 = hf + y + sw, *f1 = hf + y + 1 - sw;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int y = 2 * (lane + 32 * u) - off;
-        // 0x4B00xxxx is 2^23 + xxxx: the pixel as a float, exactly
-        const unsigned p0 = swap ? 0x7632 : 0x7610, p1 = swap ? 0x7610 : 0x7632;
-        const int y0 = y + (swap ? 1 : 0), y1 = y + (swap ? 0 : 1);
-        const float2 m = make_float2(8388608.f, 8388608.f);
-        const float2 v0 = psub(make_float2(__uint_as_float(__byte_perm(a[u], 0x4B000000u, p0)),
-                                           __uint_as_float(__byte_perm(b[u], 0x4B000000u, p0))), m);
-        const float2 v1 = psub(make_float2(__uint_as_float(__byte_perm(a[u], 0x4B000000u, p1)),
-                                           __uint_as_float(__byte_perm(b[u], 0x4B000000u, p1))), m);
-        if (y0 >= 0 && y0 < n) dst[y0 * kPitch] = pmul(v0, half_over(fr ? fr + y0 : nullptr));
-        if (y1 >= 0 && y1 < n) dst[y1 * kPitch] = pmul(v1, half_over(fr ? fr + y1 : nullptr));
+        for (int u = 0; u < U; ++u)
+            if (first + 32 * u < count) {
+                d0[64 * u * kPitch] = cscale(two_pixels(a[u], b[u], p0), f0[64 * u]);
+                d1[64 * u * kPitch] = cscale(two_pixels(a[u], b[u], p1), f1[64 * u]);
+            }
+    } else if (fr) {
+        const float *f0 = fr + y + sw, *f1 = fr + y + 1 - sw;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (first + 32 * u < count) {
+                d0[64 * u * kPitch] = cscale(two_pixels(a[u], b[u], p0), half_over(f0[64 * u]));
+                d1[64 * u * kPitch] = cscale(two_pixels(a[u], b[u], p1), half_over(f1[64 * u]));
+            }
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (first + 32 * u < count) {
+                d0[64 * u * kPitch] = pmul(two_pixels(a[u], b[u], p0), 0.5f);
+                d1[64 * u * kPitch] = pmul(two_pixels(a[u], b[u], p1), 0.5f);
+            }
+    }
+    // the pixels of words that reach past the row: the first when it is a
+    // second half, the last when it is a first half
+    if (lane < 2 && (lane ? (n + off) & 1 : off)) {
+        const int e = lane ? n - 1 : 0;
+        dst[e * kPitch] = pmul(make_float2((float)ra[e], rb ? (float)rb[e] : 0.f), fr ? half_over(fr[e]) : 0.5f);
     }
 }
 template <int N>
-__device__ __forceinline__ void stage_rows(const float *ra, const float *rb, const float *fr, int n, float2 *dst,
-                                           int lane) {
+__device__ __forceinline__ void stage_rows(const float *ra, const float *rb, const float *fr, const float *hf,
+                                           int n, float2 *dst, int lane) {
     constexpr int U = (N + 31) / 32;
     float a[U], b[U];
+    ra += lane;
+    dst += lane * kPitch;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int y = lane + 32 * u;
-        a[u] = y < n ? ra[y] : 0.f;
-        b[u] = rb && y < n ? rb[y] : 0.f;
+    for (int u = 0; u < U; ++u) a[u] = lane + 32 * u < n ? ra[32 * u] : 0.f;
+    if (rb) {
+        rb += lane;
+#pragma unroll
+        for (int u = 0; u < U; ++u) b[u] = lane + 32 * u < n ? rb[32 * u] : 0.f;
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u) b[u] = 0.f;
     }
+    if (hf) {
+        hf += lane;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-        const int y = lane + 32 * u;
-        if (y < n) dst[y * kPitch] = pmul(make_float2(a[u], b[u]), half_over(fr ? fr + y : nullptr));
+        for (int u = 0; u < U; ++u)
+            if (lane + 32 * u < n) dst[32 * u * kPitch] = make_float2(a[u] * hf[32 * u], b[u] * hf[32 * u]);
+    } else if (fr) {
+        fr += lane;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (lane + 32 * u < n) dst[32 * u * kPitch] = cscale(make_float2(a[u], b[u]), half_over(fr[32 * u]));
+    } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (lane + 32 * u < n) dst[32 * u * kPitch] = pmul(make_float2(a[u], b[u]), 0.5f);
     }
 }
 
@@ -162,6 +201,16 @@ __device__ __forceinline__ void prefetch_row(const void *p, int bytes, int lane)
     for (uintptr_t c = a + 128 * lane; c < e; c += 128 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(c));
 }
 
+// What a line of a group is: planes 2k and 2k + 1 of padded row x of a tile
+struct FwdLine {
+    long long src;  // element offset of the first plane's row; -1: a row of zeros
+    int x, k;       // k < 0: no line (past the tile's last)
+    int two;        // the second plane exists
+    int fx;         // row of the flat field
+    int n;          // pixels of a row
+};
+constexpr int kFlatRows = 2;  // flat rows kept per group (a group of 16 lines spans two x from 29 planes on)
+
 template <typename T, int N>
 __global__ void __launch_bounds__(PfaK<N>::threads, 2)
 k_rows_fwd_pfa(TileGeom g, const T *__restrict__ img, const float *__restrict__ flat, float2 *__restrict__ S, FftPlan P,
@@ -170,26 +219,73 @@ k_rows_fwd_pfa(TileGeom g, const T *__restrict__ img, const float *__restrict__ 
     constexpr int H = N / 2 + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int next;
+    __shared__ FwdLine lines[2][kPfaNL];
+    __shared__ int any[2];  // the group has a line with pixels
     const PfaSmem<N> s = pfa_layout<N>(smem_raw, line_bytes<N>());
+    float *hflat = reinterpret_cast<float *>(smem_raw + line_bytes<N>() + pfa_tail_bytes<N>());  // kFlatRows x N
     float2 *A = s.T;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     constexpr int nw = K::threads / 32;
     const int l = tid % kPfaNL, q1 = tid / kPfaNL;
+    const int LT = N * zp;  // lines of a tile
+    // line i of group grp (a thread each)
+    auto describe = [&](int grp, int i) {
+        FwdLine f;
+        const int by = grp / gx, L = (grp - by * gx) * kPfaNL + i;
+        const TileDesc d = mm_tile_desc(g, g.t0 + by);
+        f.x = L / zp;
+        f.k = L < LT ? L - f.x * zp : -1;
+        f.two = 2 * f.k + 1 < g.Z;
+        const int sx = mm_map_xy(f.x, d.x == 0, d.xd, N, g.ov);
+        f.fx = d.x0 + sx;
+        f.n = d.yd;
+        f.src = sx >= 0 ? 2 * f.k * g.isz + (long long)f.fx * g.isx + d.y0 : -1;
+        return f;
+    };
     pfa_load_tables<N, false>(s, P);
     for (int i = tid; i < kPitch; i += K::threads) A[N * kPitch + i] = make_float2(0.f, 0.f);
     __syncthreads();
     for (int i = tid; i < K::N1 * K::ipad; i += K::threads) s.tout[i] *= kPitchB;
     if (tid < 8) s.out0[tid] *= kPitchB;
-    const int LT = N * zp;  // lines of a tile
-    int tile = -1;
-    TileDesc d;
-    for (int grp = blockIdx.x; grp < ngroups;) {
+    // the half reciprocals of the flat rows of a group, once per pixel: the
+    // rows of the first line's x and the next, when those are all
+    const bool shared_flat = flat && zp >= kPfaNL - 1;
+    auto keep_flat = [&](int grp) {
+        const int by = grp / gx, x0 = (grp - by * gx) * kPfaNL / zp;
+        const TileDesc d = mm_tile_desc(g, g.t0 + by);
+        for (int r = 0; r < kFlatRows; ++r) {
+            const int sx = x0 + r < N ? mm_map_xy(x0 + r, d.x == 0, d.xd, N, g.ov) : -1;
+            if (sx < 0) continue;
+            const float *fr = flat + (long long)(d.x0 + sx) * g.fsx + d.y0;
+            for (int y = tid; y < d.yd; y += K::threads) hflat[r * N + y] = half_over(fr[y]);
+        }
+    };
+    auto describe_all = [&](int grp, int b) {  // warp 0
+        if (tid >= 32) return;
+        bool has = false;
+        if (tid < kPfaNL) {
+            const FwdLine f = describe(grp, tid);
+            lines[b][tid] = f;
+            has = f.src >= 0 && f.k >= 0;
+        }
+        has = __any_sync(0xffffffffu, has);
+        if (tid == 0) any[b] = has;
+    };
+    if ((int)blockIdx.x < ngroups) {
+        describe_all(blockIdx.x, 0);
+        if (shared_flat) keep_flat(blockIdx.x);
+    }
+    int tile = -1, buf = 0, yd = 0, y0 = 0;
+    __syncthreads();
+    for (int grp = blockIdx.x; grp < ngroups; buf ^= 1) {
         const int asked = tid == 0 ? queue_ask(queue, grp) : 0;
-        const int by = grp / gx, L0 = (grp - by * gx) * kPfaNL;
+        const int by = grp / gx;
         if (by != tile) {
             // the input table of this tile: padded column -> staged pixel
             tile = by;
-            d = mm_tile_desc(g, g.t0 + by);
+            const TileDesc d = mm_tile_desc(g, g.t0 + by);
+            yd = d.yd;
+            y0 = d.y0;
             for (int i = tid; i < K::N1 * K::ipad; i += K::threads) {
                 const int m = mm_map_xy(P.pfa_idx[i], d.y == 0, d.yd, N, g.ov);
                 s.tin[i] = (m < 0 ? N : m) * kPitchB;
@@ -199,75 +295,59 @@ k_rows_fwd_pfa(TileGeom g, const T *__restrict__ img, const float *__restrict__ 
                 s.in0[tid] = (m < 0 ? N : m) * kPitchB;
             }
         }
-        const int Lend = min(L0 + kPfaNL, LT);
+        const FwdLine *ln = lines[buf];
         float2 *Sb = S + (long long)by * g.Z * N * H;
-        bool zero = true;
-        for (int x = L0 / zp; x <= (Lend - 1) / zp; ++x) zero = zero && mm_map_xy(x, d.x == 0, d.xd, N, g.ov) < 0;
-        if (zero) {
-            // padded rows beyond the reflected data of a thin tile
-            // (deconvolver.py:135-137) transform to zero
-            for (int L = L0 + warp; L < Lend; L += nw) {
-                const int x = L / zp, k = L - x * zp;
-                for (int z = 2 * k; z < min(2 * k + 2, g.Z); ++z)
-                    for (int e = lane; e < H; e += 32) Sb[((long long)z * N + x) * H + e] = make_float2(0.f, 0.f);
+        const bool zero = !any[buf];
+        if (!zero)
+            for (int q = warp; q < kPfaNL; q += nw) {
+                const long long src = ln[q].src;
+                float2 *dst = A + q;
+                if (src >= 0 && ln[q].k >= 0)
+                    stage_rows<N>(img + src, ln[q].two ? img + src + g.isz : nullptr,
+                                  flat ? flat + ln[q].fx * g.fsx + y0 : nullptr,
+                                  shared_flat ? hflat + (ln[q].x - ln[0].x) * N : nullptr, yd, dst, lane);
+                else
+                    for (int y = lane; y < yd; y += 32) dst[y * kPitch] = make_float2(0.f, 0.f);
             }
-            if (tid == 0) next = asked;
-            __syncthreads();
-            grp = next;
-            __syncthreads();
-            continue;
-        }
-        for (int q = warp; q < kPfaNL; q += nw) {
-            const int L = L0 + q;
-            float2 *dst = A + q;
-            const T *ra = nullptr, *rb = nullptr;
-            const float *fr = nullptr;
-            if (L < LT) {
-                const int x = L / zp, k = L - x * zp;
-                const int sx = mm_map_xy(x, d.x == 0, d.xd, N, g.ov);
-                if (sx >= 0) {
-                    ra = img + 2 * k * g.isz + (long long)(d.x0 + sx) * g.isx + d.y0;
-                    if (2 * k + 1 < g.Z) rb = ra + g.isz;
-                    if (flat) fr = flat + (long long)(d.x0 + sx) * g.fsx + d.y0;
-                }
-            }
-            if (ra)
-                stage_rows<N>(ra, rb, fr, d.yd, dst, lane);
-            else
-                for (int y = lane; y < d.yd; y += 32) dst[y * kPitch] = make_float2(0.f, 0.f);
-        }
         if (tid == 0) next = asked;
         __syncthreads();
         grp = next;
-        if (grp < ngroups && grp / gx == by) {
-            // the next group's pixel rows into L2 (past the rows of this one:
-            // a group is 16 lines of the same or the next x)
-            const int N0 = (grp - by * gx) * kPfaNL;
-            for (int q = warp; q < kPfaNL && N0 + q < LT; q += nw) {
-                const int x = (N0 + q) / zp, k = N0 + q - x * zp;
-                const int sx = mm_map_xy(x, d.x == 0, d.xd, N, g.ov);
-                if (sx < 0) continue;
-                const T *ra = img + 2 * k * g.isz + (long long)(d.x0 + sx) * g.isx + d.y0;
-                prefetch_row(ra, d.yd * (int)sizeof(T), lane);
-                if (2 * k + 1 < g.Z) prefetch_row(ra + g.isz, d.yd * (int)sizeof(T), lane);
-            }
+        if (grp < ngroups) describe_all(grp, buf ^ 1);
+        if (!zero) {
+            float2 v[K::C][K::N2], x0[K::C];
+            pfa_take<N>(s, v, x0, q1, l);
+            pfa_lines<N, false>(s, v, x0, q1, l);
         }
-        float2 v[K::C][K::N2], x0[K::C];
-        pfa_take<N>(s, v, x0, q1, l);
-        pfa_lines<N, false>(s, v, x0, q1, l);
         __syncthreads();
-        // the two real rows' half spectra of each line
+        if (grp < ngroups) {
+            // the next group's pixel rows into L2
+            for (int q = warp; q < kPfaNL; q += nw) {
+                const FwdLine &f = lines[buf ^ 1][q];
+                if (f.src < 0 || f.k < 0) continue;
+                prefetch_row(img + f.src, f.n * (int)sizeof(T), lane);
+                if (f.two) prefetch_row(img + f.src + g.isz, f.n * (int)sizeof(T), lane);
+            }
+            if (shared_flat) keep_flat(grp);
+        }
+        // the two real rows' half spectra of each line; padded rows beyond the
+        // reflected data of a thin tile (deconvolver.py:135-137) are zero
         for (int q = warp; q < kPfaNL; q += nw) {
-            const int L = L0 + q;
-            if (L >= LT) break;
-            const int x = L / zp, k = L - x * zp;
-            float2 *d0 = Sb + ((long long)(2 * k) * N + x) * H, *d1 = d0 + (long long)N * H;
-            const bool two = 2 * k + 1 < g.Z;
-#pragma unroll 4
-            for (int e = lane; e < H; e += 32) {
-                const float2 ck = A[e * kPitch + q], cn = A[(e == 0 ? 0 : N - e) * kPitch + q];
-                d0[e] = make_float2(ck.x + cn.x, ck.y - cn.y);
-                if (two) d1[e] = make_float2(ck.y + cn.y, cn.x - ck.x);
+            if (ln[q].k < 0) break;
+            float2 *d0 = Sb + ((long long)(2 * ln[q].k) * N + ln[q].x) * H + lane, *d1 = d0 + (long long)N * H;
+            const bool two = ln[q].two;
+            const float2 *lo = A + lane * kPitch + q, *hi = A + (N - lane) * kPitch + q;
+#pragma unroll
+            for (int u = 0; u < (H + 31) / 32; ++u) {
+                if (lane + 32 * u >= H) continue;
+                float2 a = make_float2(0.f, 0.f), b = a;
+                if (!zero) {
+                    // element N is element 0
+                    const float2 ck = lo[32 * u * kPitch], cn = u == 0 && lane == 0 ? ck : hi[-32 * u * kPitch];
+                    a = make_float2(ck.x + cn.x, ck.y - cn.y);
+                    b = make_float2(ck.y + cn.y, cn.x - ck.x);
+                }
+                d0[32 * u] = a;
+                if (two) d1[32 * u] = b;
             }
         }
         __syncthreads();
@@ -286,6 +366,13 @@ k_rows_fwd_pfa(TileGeom g, const T *__restrict__ img, const float *__restrict__ 
 // ---------------------------------------------------------------------------
 constexpr int kMaxWinTiles = 256;
 
+// What a line of a group is: rows `row` and row + 1 of the batch
+struct InvLine {
+    long long row;
+    int z, x;   // plane and first row in it (windows); z < 0: no line
+    int store;  // bit 0: the first row is stored, bit 1: the second
+};
+
 template <int N, bool WIN>
 __global__ void __launch_bounds__(PfaK<N>::threads, 2)
 k_rows_inv_pfa(const float2 *__restrict__ S, long long nrows, TileGeom g, int reach, float *__restrict__ out,
@@ -296,6 +383,7 @@ k_rows_inv_pfa(const float2 *__restrict__ S, long long nrows, TileGeom g, int re
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int next;
     __shared__ int cum[WIN ? kMaxWinTiles + 1 : 1];  // groups before tile t
+    __shared__ InvLine lines[2][kPfaNL];
     const PfaSmem<N> s = pfa_layout<N>(smem_raw, line_bytes<N>());
     float *rtab = reinterpret_cast<float *>(smem_raw + line_bytes<N>() + pfa_tail_bytes<N>());  // 1 / window count
     float2 *A = s.T;
@@ -321,81 +409,79 @@ k_rows_inv_pfa(const float2 *__restrict__ S, long long nrows, TileGeom g, int re
     for (int i = tid; i < 2 * K::N1 * K::ipad + 16; i += K::threads) s.tin[i] *= kPitchB;
     __syncthreads();
     const int ngroups = WIN ? cum[g.nt] : (int)((nrows / 2 + kPfaNL - 1) / kPfaNL);
-    int t = 0;
-    for (int grp = blockIdx.x; grp < ngroups;) {
-        const int asked = tid == 0 ? queue_ask(queue, grp) : 0;
-        // line q of the group: rows row(q) and row(q) + 1 of the batch (the
-        // first one even); nl lines exist
-        int xlo = 0, xhi = N, ylo = 0, yhi = N, np = 0, nl, L0;
-        long long tbase = 0;
+    // line i of group grp (a thread each), t: a tile at or before the group's
+    auto describe = [&](int grp, int i, int t) {
+        InvLine f;
         if constexpr (WIN) {
             while (cum[t + 1] <= grp) ++t;
+            int xlo, xhi, ylo, yhi;
             read_window(g, t, reach, xlo, xhi, ylo, yhi);
-            np = (xhi - (xlo & ~1) + 1) / 2;
-            L0 = (grp - cum[t]) * kPfaNL;
-            nl = min(kPfaNL, g.Z * np - L0);
-            tbase = (long long)t * g.Z * N;
+            const int np = (xhi - (xlo & ~1) + 1) / 2, L = (grp - cum[t]) * kPfaNL + i;
+            f.z = L < g.Z * np ? L / np : -1;
+            f.x = (xlo & ~1) + 2 * (L - L / np * np);
+            f.row = ((long long)t * g.Z + f.z) * N + f.x;
+            f.store = (f.x >= xlo ? 1 : 0) | (f.x + 1 < xhi ? 2 : 0);
         } else {
-            L0 = grp * kPfaNL;
-            nl = (int)min((long long)kPfaNL, nrows / 2 - L0);
+            f.row = 2LL * (grp * kPfaNL + i);
+            f.z = f.row < nrows ? 0 : -1;
+            f.x = 0;
+            f.store = 3;
         }
-        // plane and first row (in its plane) of line q
-        auto line_at = [&](int q, int &z, int &x) {
-            z = WIN ? (L0 + q) / np : 0;
-            x = WIN ? (xlo & ~1) + 2 * (L0 + q - z * np) : 0;
-        };
-        auto row_of = [&](int q, int z, int x) { return WIN ? tbase + (long long)z * N + x : 2LL * (L0 + q); };
-        for (int q = warp; q < nl; q += nw) {
-            int z, x;
-            line_at(q, z, x);
-            const float2 *r0 = S + row_of(q, z, x) * H, *r1 = r0 + H;
-            constexpr int U = 4;
-            for (int k0 = lane; k0 < H; k0 += 32 * U) {
-                float2 a[U], b[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int k = k0 + 32 * u;
-                    a[u] = b[u] = make_float2(0.f, 0.f);
-                    if (k < H) {
-                        a[u] = __ldcs(r0 + k);
-                        b[u] = __ldcs(r1 + k);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const int k = k0 + 32 * u;
-                    if (k >= H) break;
-                    if (k == 0 || k == N / 2) {
-                        A[k * kPitch + q] = make_float2(a[u].x, b[u].x);
-                    } else {
-                        A[k * kPitch + q] = make_float2(a[u].x - b[u].y, a[u].y + b[u].x);
-                        A[(N - k) * kPitch + q] = make_float2(a[u].x + b[u].y, b[u].x - a[u].y);
-                    }
-                }
+        return f;
+    };
+    int t = 0, buf = 0, ylo = 0, yhi = N, t_known = -1;
+    if ((int)blockIdx.x < ngroups && tid < kPfaNL) lines[0][tid] = describe(blockIdx.x, tid, 0);
+    __syncthreads();
+    for (int grp = blockIdx.x; grp < ngroups; buf ^= 1) {
+        const int asked = tid == 0 ? queue_ask(queue, grp) : 0;
+        if constexpr (WIN) {
+            while (cum[t + 1] <= grp) ++t;
+            if (t != t_known) {
+                int xlo, xhi;
+                read_window(g, t, reach, xlo, xhi, ylo, yhi);
+                t_known = t;
             }
+        }
+        const InvLine *ln = lines[buf];
+        for (int q = warp; q < kPfaNL; q += nw) {
+            if (ln[q].z < 0) break;
+            const float2 *r0 = S + ln[q].row * H, *r1 = r0 + H;
+            // frequencies 1 .. N/2 - 1 give two elements each, all loads first;
+            // 0 and N/2 one
+            constexpr int U = (H - 2 + 31) / 32;
+            float2 a[U], b[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (lane + 32 * u < H - 2) {
+                    a[u] = __ldcs(r0 + 1 + lane + 32 * u);
+                    b[u] = __ldcs(r1 + 1 + lane + 32 * u);
+                }
+            float2 *lo = A + (1 + lane) * kPitch + q, *hi = A + (N - 1 - lane) * kPitch + q;
+            if (lane < 2) A[lane * (N / 2) * kPitch + q] = make_float2(r0[lane * (N / 2)].x, r1[lane * (N / 2)].x);
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (lane + 32 * u < H - 2) {
+                    lo[32 * u * kPitch] = make_float2(a[u].x - b[u].y, a[u].y + b[u].x);
+                    hi[-32 * u * kPitch] = make_float2(a[u].x + b[u].y, b[u].x - a[u].y);
+                }
         }
         if (tid == 0) next = asked;
         __syncthreads();
         grp = next;
-        if (!WIN || grp < cum[t + 1]) {
-            // the next group's spectrum rows into L2
-            const int N0 = WIN ? (grp - cum[t]) * kPfaNL : grp * kPfaNL;
-            const long long end = WIN ? (long long)g.Z * np : nrows / 2;
-            for (int q = warp; q < kPfaNL && N0 + q < end; q += nw) {
-                const int z = WIN ? (N0 + q) / np : 0;
-                const long long row = WIN ? tbase + (long long)z * N + (xlo & ~1) + 2 * (N0 + q - z * np) : 2LL * (N0 + q);
-                prefetch_row(S + row * H, 2 * H * 8, lane);
-            }
-        }
+        if (grp < ngroups && tid < kPfaNL) lines[buf ^ 1][tid] = describe(grp, tid, t);
         float2 v[K::C][K::N2], x0[K::C];
         pfa_take<N>(s, v, x0, q1, l);
         pfa_lines<N, true>(s, v, x0, q1, l);
         __syncthreads();
-        for (int q = warp; q < nl; q += nw) {
-            int z, x;
-            line_at(q, z, x);
-            const long long r0 = row_of(q, z, x);
-            const bool first = !WIN || x >= xlo, second = !WIN || x + 1 < xhi;
+        if (grp < ngroups)
+            // the next group's spectrum rows into L2
+            for (int q = warp; q < kPfaNL && lines[buf ^ 1][q].z >= 0; q += nw)
+                prefetch_row(S + lines[buf ^ 1][q].row * H, 2 * H * 8, lane);
+        for (int q = warp; q < kPfaNL; q += nw) {
+            if (ln[q].z < 0) break;
+            const int z = ln[q].z, x = ln[q].x;
+            const long long r0 = ln[q].row;
+            const bool first = ln[q].store & 1, second = ln[q].store & 2;
             if (WIN && stitch) {
                 // the FOV voxels whose last writer in the reference's order is
                 // this tile (Deconvolver.apply, deconvolver.py:179-183)
@@ -415,11 +501,19 @@ k_rows_inv_pfa(const float2 *__restrict__ S, long long nrows, TileGeom g, int re
                 continue;
             }
             float *o0 = out + r0 * N, *o1 = o0 + N;
-#pragma unroll 4
-            for (int e = ylo + lane; e < yhi; e += 32) {
-                const float2 w = A[e * kPitch + q];
-                if (first) o0[e] = w.x;
-                if (second) o1[e] = w.y;
+            if (first && second) {
+#pragma unroll 8
+                for (int e = ylo + lane; e < yhi; e += 32) {
+                    const float2 w = A[e * kPitch + q];
+                    o0[e] = w.x;
+                    o1[e] = w.y;
+                }
+            } else {
+                for (int e = ylo + lane; e < yhi; e += 32) {
+                    const float2 w = A[e * kPitch + q];
+                    if (first) o0[e] = w.x;
+                    if (second) o1[e] = w.y;
+                }
             }
             if (WIN || delta < 0) continue;
             // y box mean of both rows: each lane slides a window along a
@@ -471,8 +565,8 @@ int launch_fwd(const TileGeom &g, const void *img, const float *flat, float2 *S,
     TileGeom ga = g;
     FftPlan Pa = P;
     void *args[] = {&ga, &img, &flat, &S, &Pa, &zp, &gx, &ngroups, &queue};
-    return launch_fft_kernel((const void *)k_rows_fwd_pfa<T, N>, dim3(fft_grid(ngroups, {K::threads, 2})), rows_smem<N>(),
-                             st, args, K::threads);
+    return launch_fft_kernel((const void *)k_rows_fwd_pfa<T, N>, dim3(fft_grid(ngroups, {K::threads, 2})),
+                             rows_smem<N>() + sizeof(float) * kFlatRows * N, st, args, K::threads);
 }
 
 template <int N, bool WIN>
