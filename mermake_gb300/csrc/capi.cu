@@ -232,14 +232,18 @@ int fill_geom(TileGeom &g, int Z, int X, int Y, long long isz, long long isx, lo
 // _DIRECT (k_zconv) or _TRANSFORMS (k_zpass).  The context's MM_OPT_ZFORM
 // choice when the batch qualifies for it (a z kernel, one spectrum for the
 // shared and tensor forms, the forms' shape limits), else the first of
-// registers, shared, direct and transforms that qualifies, the shared-spectrum
-// matrix forms only for batches of at least MM_ZOP_MIN_TILES tiles.  A
+// registers, shared, direct and transforms that qualifies, the shared-memory
+// matrix form only for batches of at least MM_ZOP_MIN_TILES tiles.  A
 // register-form batch split into tile chunks (deeper tiles: each chunk reloads
 // the z kernel and rounds its tiles up to whole thread groups) gives way to
 // the shared-memory form where that form takes the depth.
 bool zth_takes(const TileGeom &g, bool forced) {
-    if (g.npsf != 1 || g.nt < (forced ? 1 : MM_ZOP_MIN_TILES)) return false;
-    const int chunks = mm_zth_supported(g.Z, g.zpad, g.nt, (long long)g.P * g.H);
+    if (g.npsf != 1) return false;
+    const long long plane = (long long)g.P * g.H;
+    // one tile shares no matrix: the per-tile form has the wider rows (0.12
+    // against 0.15 ms at Z = 40, P = 678)
+    if (g.nt == 1 && !forced && mm_zpt_supported(g.Z, g.zpad, 1, plane)) return false;
+    const int chunks = mm_zth_supported(g.Z, g.zpad, g.nt, plane);
     return chunks == 1 || (chunks > 1 && (forced || mm_zop_supported(g.Z, g.zpad) == 0));
 }
 
@@ -253,9 +257,9 @@ int zform_of(const mm_ctx *c, const TileGeom &g, const float2 *zop) {
                 if (!zop) return false;
                 // one spectrum and a batch the shared-spectrum forms take: the
                 // per-tile form only where k_zth_apply does not take it
-                if (g.npsf == 1 && g.nt >= min_tiles && mm_zop_supported(g.Z, g.zpad) != 0)
-                    return zth_takes(g, forced);
-                return zth_takes(g, forced) || mm_zpt_supported(g.Z, g.zpad, g.nt, plane) != 0;
+                if (zth_takes(g, forced)) return true;
+                if (g.npsf == 1 && g.nt >= min_tiles && mm_zop_supported(g.Z, g.zpad) != 0) return false;
+                return mm_zpt_supported(g.Z, g.zpad, g.nt, plane) != 0;
             }
             case MM_ZFORM_SHARED:
                 return zop && g.npsf == 1 && g.nt >= min_tiles && mm_zop_supported(g.Z, g.zpad) != 0;

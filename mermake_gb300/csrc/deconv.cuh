@@ -153,10 +153,11 @@ int mm_launch_zpass(const TileGeom &g, float2 *S, const float2 *W, long long wst
 // W along z (zop.cu): as a matrix per frequency over a batch that shares one
 // spectrum (mm_launch_zop_apply), or as the direct sum per tile
 // (mm_launch_zconv).
-// The matrix form's CTAs shrink with the batch (threads = 4 frequencies x
-// ceil(Z / 5) row groups x ceil(nt / 5) tile groups), so a launch costs nearly
-// as much for 10 tiles as for 25 (3.5 against 3.9 ms at Z = 50, P = 678);
-// batches of fewer tiles than this take the direct sum.
+// The shared-memory matrix form's CTAs shrink with the batch (threads = 4
+// frequencies x ceil(Z / 5) row groups x ceil(nt / 5) tile groups), so a launch
+// costs nearly as much for 10 tiles as for 25 (3.5 against 3.9 ms at Z = 50, P =
+// 678); where the register form takes no batch of the shape, batches of fewer
+// tiles than this take the direct sum.
 #define MM_ZOP_MIN_TILES 10
 #define MM_ZOP_MAX_Z 64
 #define MM_ZOP_MAX_ZP 400
@@ -172,7 +173,7 @@ int mm_launch_zconv(float2 *S, const float2 *w, long long wstride, int Z, int zp
                     int nt, int npsf, const float *fresp, cudaStream_t st);
 // The z operator with the matrix of each frequency formed in registers from
 // the z kernel (Toeplitz plus two masked Hankel parts, 1 <= zpad <= Z - 1,
-// Z a multiple of 5) and its operands staged by TMA (zop_tma.cu).  A CTA that
+// 2 <= Z <= 128) and its operands staged asynchronously (zop_tma.cu).  A CTA that
 // gives up waiting for its copies sets *err.  mm_zth_supported returns the
 // number of tile chunks a batch of nt tiles is split into (0: not supported).
 int mm_zth_supported(int Z, int zpad, int nt, long long plane);

@@ -71,11 +71,6 @@ __device__ __forceinline__ void copy16s(unsigned dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 
-__device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c) {
-    c.x = fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x));
-    c.y = fmaf(a.x, b.y, fmaf(a.y, b.x, c.y));
-    return c;
-}
 
 struct ZptArgs {
     int Z, Zp, nt, t0, npsf;
@@ -106,6 +101,32 @@ constexpr int zpt_block(int Z, int ntpi, int pb) { return (pb * (Z / kTI) * ntpi
 struct Rings {
     float2 rT[kTI], rH[kTI], acc[kTI];
 };
+// column of matrix entries (direct + reflected, u = j mod 5) times x.  ONE (one
+// PSF): the order of products of zop_tma.cu, so that a tile's result is the same
+// bits in both; else row by row, which is 2 % faster (64 tiles of Z = 40, P =
+// 478: 3.38 against 3.45 ms)
+template <bool ONE>
+__device__ __forceinline__ void col_products(Rings &R, float2 x, int u) {
+    float2 m[kTI];
+#pragma unroll
+    for (int q = 0; q < kTI; ++q) m[q] = cadd(R.rT[(q - u + kTI) % kTI], R.rH[(q + u) % kTI]);
+    if constexpr (ONE) {
+#pragma unroll
+        for (int q = 0; q < kTI; ++q) R.acc[q].x = fmaf(m[q].x, x.x, R.acc[q].x);
+#pragma unroll
+        for (int q = 0; q < kTI; ++q) R.acc[q].y = fmaf(m[q].y, x.x, R.acc[q].y);
+#pragma unroll
+        for (int q = 0; q < kTI; ++q) R.acc[q].x = fmaf(-m[q].y, x.y, R.acc[q].x);
+#pragma unroll
+        for (int q = 0; q < kTI; ++q) R.acc[q].y = fmaf(m[q].x, x.y, R.acc[q].y);
+    } else {
+#pragma unroll
+        for (int q = 0; q < kTI; ++q) {
+            R.acc[q].x = fmaf(m[q].x, x.x, fmaf(-m[q].y, x.y, R.acc[q].x));
+            R.acc[q].y = fmaf(m[q].x, x.y, fmaf(m[q].y, x.x, R.acc[q].y));
+        }
+    }
+}
 template <int PB>
 __device__ __forceinline__ void ring_start(Rings &R, const float2 *W, int i0, int kb, int hrow) {
 #pragma unroll
@@ -115,18 +136,16 @@ __device__ __forceinline__ void ring_start(Rings &R, const float2 *W, int i0, in
     R.rT[0] = R.rH[kTI - 1] = make_float2(0.f, 0.f);
 }
 // column j, u = j mod 5
-template <int PB>
+template <int PB, bool ONE>
 __device__ __forceinline__ void col_u(Rings &R, const float2 *W, const float2 *xr, int i0, int j, int kb, int hrow,
                                       int u) {
     R.rT[(kTI - u) % kTI] = W[(i0 - j + kb) * PB];
     R.rH[(u + kTI - 1) % kTI] = W[(i0 + j + kTI - 1 + hrow) * PB];
-    const float2 x = xr[(size_t)j * PB];
-#pragma unroll
-    for (int q = 0; q < kTI; ++q) R.acc[q] = cfma(cadd(R.rT[(q - u + kTI) % kTI], R.rH[(q + u) % kTI]), x, R.acc[q]);
+    col_products<ONE>(R, xr[(size_t)j * PB], u);
 }
-template <int PB, int U>
+template <int PB, int U, bool ONE>
 __device__ __forceinline__ void col(Rings &R, const float2 *W, const float2 *xr, int i0, int j, int kb, int hrow) {
-    col_u<PB>(R, W, xr, i0, j, kb, hrow, U);
+    col_u<PB, ONE>(R, W, xr, i0, j, kb, hrow, U);
 }
 // a column that starts a class: the reflected ring from its source
 template <int PB, int U>
@@ -137,14 +156,12 @@ __device__ __forceinline__ void reload(Rings &R, const float2 *W, int i0, int j,
 
 // a column of the class with both reflections, its reflected value summed
 // from the two kernel rows (kb: w[0], ko: w[-(2Z-2)])
-template <int PB, int U>
+template <int PB, int U, bool ONE>
 __device__ __forceinline__ void col2(Rings &R, const float2 *W, const float2 *xr, int i0, int j, int kb, int ko) {
     R.rT[(kTI - U) % kTI] = W[(i0 - j + kb) * PB];
     const int h = i0 + j + kTI - 1;
     R.rH[(U + kTI - 1) % kTI] = cadd(W[(h + kb) * PB], W[(h + ko) * PB]);
-    const float2 x = xr[(size_t)j * PB];
-#pragma unroll
-    for (int q = 0; q < kTI; ++q) R.acc[q] = cfma(cadd(R.rT[(q - U + kTI) % kTI], R.rH[(q + U) % kTI]), x, R.acc[q]);
+    col_products<ONE>(R, xr[(size_t)j * PB], U);
 }
 template <int PB, int U>
 __device__ __forceinline__ void reload2(Rings &R, const float2 *W, int i0, int j, int kb, int ko) {
@@ -152,7 +169,7 @@ __device__ __forceinline__ void reload2(Rings &R, const float2 *W, int i0, int j
     for (int q = 0; q < kTI - 1; ++q) R.rH[(q + U) % kTI] = cadd(W[(i0 + j + q + kb) * PB], W[(i0 + j + q + ko) * PB]);
 }
 
-template <int ZC, bool FULL, int PB>
+template <int ZC, bool FULL, int PB, bool ONE>
 __global__ void __launch_bounds__(kMaxCompute + 32 * kProd, 2)
 k_zpt_apply(float2 *__restrict__ S, const float2 *__restrict__ w, const ZptArgs a) {
     constexpr int kPB = PB;          // frequencies per item
@@ -294,26 +311,26 @@ k_zpt_apply(float2 *__restrict__ S, const float2 *__restrict__ w, const ZptArgs 
                 // 1 .. Z - 2 the sum w[i + j] + w[i + j - 2Z + 2] (two loads
                 // and an add per column), column Z - 1 w[i + j]
                 ring_start<PB>(R, Wp, i0, kb, ko);
-                col<PB, 0>(R, Wp, xr, i0, 0, kb, ko);
+                col<PB, 0, ONE>(R, Wp, xr, i0, 0, kb, ko);
                 reload2<PB, 1>(R, Wp, i0, 1, kb, ko);
-                col2<PB, 1>(R, Wp, xr, i0, 1, kb, ko);
-                col2<PB, 2>(R, Wp, xr, i0, 2, kb, ko);
-                col2<PB, 3>(R, Wp, xr, i0, 3, kb, ko);
-                col2<PB, 4>(R, Wp, xr, i0, 4, kb, ko);
+                col2<PB, 1, ONE>(R, Wp, xr, i0, 1, kb, ko);
+                col2<PB, 2, ONE>(R, Wp, xr, i0, 2, kb, ko);
+                col2<PB, 3, ONE>(R, Wp, xr, i0, 3, kb, ko);
+                col2<PB, 4, ONE>(R, Wp, xr, i0, 4, kb, ko);
                 for (int j0 = kTI; j0 < Z - kTI; j0 += kTI) {
-                    col2<PB, 0>(R, Wp, xr, i0, j0, kb, ko);
-                    col2<PB, 1>(R, Wp, xr, i0, j0 + 1, kb, ko);
-                    col2<PB, 2>(R, Wp, xr, i0, j0 + 2, kb, ko);
-                    col2<PB, 3>(R, Wp, xr, i0, j0 + 3, kb, ko);
-                    col2<PB, 4>(R, Wp, xr, i0, j0 + 4, kb, ko);
+                    col2<PB, 0, ONE>(R, Wp, xr, i0, j0, kb, ko);
+                    col2<PB, 1, ONE>(R, Wp, xr, i0, j0 + 1, kb, ko);
+                    col2<PB, 2, ONE>(R, Wp, xr, i0, j0 + 2, kb, ko);
+                    col2<PB, 3, ONE>(R, Wp, xr, i0, j0 + 3, kb, ko);
+                    col2<PB, 4, ONE>(R, Wp, xr, i0, j0 + 4, kb, ko);
                 }
                 const int j0 = Z - kTI;
-                col2<PB, 0>(R, Wp, xr, i0, j0, kb, ko);
-                col2<PB, 1>(R, Wp, xr, i0, j0 + 1, kb, ko);
-                col2<PB, 2>(R, Wp, xr, i0, j0 + 2, kb, ko);
-                col2<PB, 3>(R, Wp, xr, i0, j0 + 3, kb, ko);
+                col2<PB, 0, ONE>(R, Wp, xr, i0, j0, kb, ko);
+                col2<PB, 1, ONE>(R, Wp, xr, i0, j0 + 1, kb, ko);
+                col2<PB, 2, ONE>(R, Wp, xr, i0, j0 + 2, kb, ko);
+                col2<PB, 3, ONE>(R, Wp, xr, i0, j0 + 3, kb, ko);
                 reload<PB, 4>(R, Wp, i0, j0 + 4, kb);
-                col<PB, 4>(R, Wp, xr, i0, j0 + 4, kb, kb);
+                col<PB, 4, ONE>(R, Wp, xr, i0, j0 + 4, kb, kb);
             } else {
                 auto seg_row = [&](int k) {
                     const int cls = a.segc[k];
@@ -332,7 +349,7 @@ k_zpt_apply(float2 *__restrict__ S, const float2 *__restrict__ w, const ZptArgs 
 #pragma unroll
                             for (int q = 0; q < kTI - 1; ++q) R.rH[(q + u) % kTI] = Wp[(i0 + j + q + hrow) * kPB];
                         }
-                        col_u<PB>(R, Wp, xr, i0, j, kb, hrow, u);
+                        col_u<PB, ONE>(R, Wp, xr, i0, j, kb, hrow, u);
                     }
                 }
             }
@@ -402,6 +419,16 @@ int zpt_config(int Z, bool full, int *pb) {
     return 0;
 }
 
+template <bool ONE>
+const void *zpt_kernel(int Z, bool full, int pb) {
+    if (pb == 16)
+        return !full     ? (const void *)k_zpt_apply<0, false, 16, ONE>
+               : Z == 40 ? (const void *)k_zpt_apply<40, true, 16, ONE>
+               : Z == 50 ? (const void *)k_zpt_apply<50, true, 16, ONE>
+                         : (const void *)k_zpt_apply<0, true, 16, ONE>;
+    return full ? (const void *)k_zpt_apply<0, true, 8, ONE> : (const void *)k_zpt_apply<0, false, 8, ONE>;
+}
+
 }  // namespace
 
 int mm_zpt_supported(int Z, int zpad, int nt, long long plane) {
@@ -452,14 +479,7 @@ int mm_launch_zpt_apply(float2 *S, const float2 *w, long long wstride, int Z, in
     a.err = err;
     const size_t sm = zpt_smem(Z, a.ntpi, pb, full);
     const int threads = zpt_block(Z, a.ntpi, pb);
-    const void *fn;
-    if (pb == 16)
-        fn = !full     ? (const void *)k_zpt_apply<0, false, 16>
-             : Z == 40 ? (const void *)k_zpt_apply<40, true, 16>
-             : Z == 50 ? (const void *)k_zpt_apply<50, true, 16>
-                       : (const void *)k_zpt_apply<0, true, 16>;
-    else
-        fn = full ? (const void *)k_zpt_apply<0, true, 8> : (const void *)k_zpt_apply<0, false, 8>;
+    const void *fn = npsf == 1 ? zpt_kernel<true>(Z, full, pb) : zpt_kernel<false>(Z, full, pb);
     if (int rc = mm_set_smem(fn, sm)) return rc;
     int per_sm = 0;
     MM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, sm));

@@ -11,22 +11,30 @@
 //   M[i][j] = w[i - j] + [1 <= j <= zpad] w[i + j] + [Z-1-zpad <= j <= Z-2] w[i + j - 2Z + 2]:
 //
 // a Toeplitz matrix plus two masked Hankel matrices.  A thread owns rows
-// i0 .. i0 + 4 of kTT tiles; along j each family's five values slide by one
-// place, so the thread keeps them in three register rings of five and loads
-// one new value of each per column (the slots are compile-time constants with
-// j unrolled by five).  No matrix is stored: shared memory holds only the
-// operands, X (nt x Z x kPB: 32-byte rows, copied by cp.async) and the kernel
-// rows w[-kA .. 2Z-2] (two TMA boxes of the (Zp, plane) kernel, the negative
-// rows from its top; kA is 2Z - 2 rounded up to a multiple of four, so that
-// both boxes land on 128-byte boundaries as tiled TMA requires), double
-// buffered.  The persistent CTAs take groups of kPB consecutive frequencies.
-// A producer warp issues each group's copies once the buffer is free; the
-// compute warps take the group's work in warp-sized units from a shared
-// counter, wait only for their buffer to fill (its "full" mbarrier completes
-// with the copies: 32 cp.async arrivals and the TMA bytes) and release it with
-// one arrive per unit on its "empty" mbarrier, so no CTA barrier separates the
-// groups.  Every wait is bounded: a thread that gives up
-// records the failure in *err and returns.
+// i0 .. i0 + 4 of TT tiles; along j the direct values w[i - j] and the
+// reflected ones slide by one place, so the thread keeps each in a register
+// ring of five and loads one new direct value and the one or two reflected ones
+// per column (with j unrolled by five the slots are compile-time constants).
+// No matrix is stored: shared memory holds only the operands, X (nt x Z rows of
+// PB frequencies, copied by cp.async) and the kernel rows w[-kA .. 2Z-2] (two
+// TMA boxes of the (Zp, plane) kernel, the negative rows from its top; kA is
+// 2Z - 2 rounded up to a multiple of four, so that both boxes land on 128-byte
+// boundaries as tiled TMA requires), double buffered.  The persistent CTAs take
+// groups of PB consecutive frequencies.  A producer warp issues each group's
+// copies once the buffer is free; the compute warps take the group's work in
+// warp-sized units from a shared counter, wait only for their buffer to fill
+// (its "full" mbarrier completes with the copies: 32 cp.async arrivals and the
+// TMA bytes) and release it with one arrive per unit on its "empty" mbarrier,
+// so no CTA barrier separates the groups.  Every wait is bounded: a thread that
+// gives up records the failure in *err and returns.
+//
+// Every output sums its columns in ascending order with the same products
+// (k_zpt_apply's too), so a tile's result does not depend on the batch it is in.
+//
+// What bounds it: FP32 issue.  A product needs three register reads; at 25
+// tiles, Z = 50 and P = 678 the 115 GFLOP of a launch take 2.69 ms (21.4 T
+// products/s of the 40.3 T that 152 SMs have at 2.07 GHz; a loop of products
+// with two new operands each reaches 33 T).
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -36,11 +44,10 @@
 
 namespace {
 
-constexpr int kPB = 4;      // frequencies per group (32 bytes of a plane row)
-constexpr int kLPR = kPB / 2;  // 16-byte pieces of a row (copying lanes per row)
 constexpr int kTI = 5;      // rows of a thread, and the unroll of the column loop
-constexpr int kTT = 5;      // tiles of a thread
-constexpr int kThreadsMax = 256;
+// threads of a CTA at most, and CTAs per SM that the registers are shared out for
+constexpr int zth_ctas(int tt, int pb) { return tt == 5 && pb == 8 ? 1 : 2; }
+constexpr int zth_max_threads(int tt, int pb) { return tt == 5 && pb == 8 ? 448 : 256; }
 constexpr unsigned kWaitPolls = 1u << 24;
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -89,29 +96,50 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
         : "memory");
 }
 
-__device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c) {
-    c.x = fmaf(a.x, b.x, fmaf(-a.y, b.y, c.x));
-    c.y = fmaf(a.x, b.y, fmaf(a.y, b.x, c.y));
-    return c;
-}
-
+// The accumulators of a thread's kTI rows x TT tiles
+template <int TT>
+struct ZthAcc {
+    float2 v[kTI][TT];
+    __device__ __forceinline__ void clear() {
+#pragma unroll
+        for (int q = 0; q < kTI; ++q)
+#pragma unroll
+            for (int b = 0; b < TT; ++b) v[q][b] = make_float2(0.f, 0.f);
+    }
+    __device__ __forceinline__ void add(const float2 (&m)[kTI], const float2 (&x)[TT]) {
+        // an operand of each product is the previous one's: with all operands
+        // new, register reads bound the rate (a column of 25 products took 4 %
+        // longer in row order, and 10 % with the two products of x[b].x apart)
+#pragma unroll
+        for (int b = 0; b < TT; ++b) {
+#pragma unroll
+            for (int q = 0; q < kTI; ++q) v[q][b].x = fmaf(m[q].x, x[b].x, v[q][b].x);
+#pragma unroll
+            for (int q = 0; q < kTI; ++q) v[q][b].y = fmaf(m[q].y, x[b].x, v[q][b].y);
+#pragma unroll
+            for (int q = 0; q < kTI; ++q) v[q][b].x = fmaf(-m[q].y, x[b].y, v[q][b].x);
+#pragma unroll
+            for (int q = 0; q < kTI; ++q) v[q][b].y = fmaf(m[q].x, x[b].y, v[q][b].y);
+        }
+    }
+    __device__ __forceinline__ float2 get(int q, int b) const { return v[q][b]; }
+};
 struct ZthArgs {
     int Z, Zp, nt;
     int ntc;           // tiles of a chunk (the X box's height)
-    int ntg;           // tile groups of kTT a CTA computes (ceil(ntc / kTT))
+    int ntg;           // tile groups of TT a CTA computes (ceil(ntc / TT))
     int nchunks;       // chunks the batch's tiles are split into
     long long plane;
-    int nitems;        // frequency groups (ceil(plane / kPB)) x chunks
+    int nitems;        // frequency groups (ceil(plane / PB)) x chunks
     int kA;            // staged row of w[0]: 2Z - 2 rounded up to a multiple of 4
-    unsigned xbytes;   // X bytes of an item (kPB x Z x ntc float2)
-    unsigned wbytesA;  // kernel rows -kA .. -1 (kA x 32 bytes, a multiple of 128)
+    unsigned wbytesA;  // kernel rows -kA .. -1 (a multiple of 128 bytes)
     unsigned wbytesB;  // kernel rows 0 .. 2Z-2
     unsigned bufstride, woff;  // bytes per buffer, offset of the kernel rows in it
     unsigned zoff;     // bytes: the zero rows (2Z + 3 of them) after the two buffers
     // the columns j in segments of one reflection class: segment k covers
-    // [segj[k], segj[k + 1]) (segj[nseg] = Z) with class segc[k]: 0 only the
-    // reflection about zpad (w[i + j]), 1 only the one about zpad + Z - 1
-    // (w[i + j - 2Z + 2]), 2 both (hB[i + j]), 3 neither
+    // [segj[k], segj[k + 1]) (segj[nseg] = Z) with class segc[k]: bit 0 the
+    // reflection about zpad (w[i + j]), bit 1 the one about zpad + Z - 1
+    // (w[i + j - 2Z + 2])
     int nseg, segj[6], segc[6];
     const float *fresp;
     unsigned *err;
@@ -130,18 +158,20 @@ __device__ __forceinline__ void zth_item(const ZthArgs &a, int item, int &grp, i
 }
 
 // ZC > 0: Z known at compile time (50, the depth of every channel of the
-// benchmark FOV); otherwise any multiple of kTI.  CH: the batch is split
-// into several tile chunks (otherwise item == frequency group, one box of
-// all nt tiles).
-template <int ZC, bool CH>
-__global__ void __launch_bounds__(kThreadsMax, 2)
+// benchmark FOV); otherwise any depth (the last row group and the last column
+// block are cut).  TT: tiles of a thread.  PB: frequencies of a group.  CH: the
+// batch is split into several tile chunks (otherwise item == frequency group,
+// one box of all nt tiles).
+template <int ZC, int TT, int PB, bool CH>
+__global__ void __launch_bounds__(zth_max_threads(TT, PB), zth_ctas(TT, PB))
 k_zth_apply(float2 *__restrict__ S, const __grid_constant__ CUtensorMap wmapA, const __grid_constant__ CUtensorMap wmapB, const ZthArgs a) {
+    constexpr int kLPR = PB / 2;  // 16-byte pieces of a row (copying lanes per row)
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) uint64_t full[2], empty[2], wfull[2];
+    __shared__ __align__(8) uint64_t full[2], empty[2];
     __shared__ int3 item_of[2];  // (group, first owned tile, box start) of each buffer's item
     __shared__ unsigned unit_next;  // the next (item, warp unit) a compute warp takes
     const int Z = ZC > 0 ? ZC : a.Z;
-    const int nig = Z / kTI;
+    const int nig = (Z + kTI - 1) / kTI;
     const int tid = threadIdx.x;
     const int kb = a.kA;              // row of w[0] in the staged kernel rows
     const int ko = kb - (2 * Z - 2);  // row of w[-(2Z-2)], the lowest index the rings read
@@ -154,28 +184,27 @@ k_zth_apply(float2 *__restrict__ S, const __grid_constant__ CUtensorMap wmapA, c
         return;
     }
     const int lane = tid & 31, warp = tid >> 5;
-    const int ncw = (kPB * nig * a.ntg + 31) / 32;  // compute warps; warp ncw produces
+    const int ncw = (PB * nig * a.ntg + 31) / 32;  // compute warps; warp ncw produces
     if (tid == 0) {
         for (int b = 0; b < 2; ++b) {
-            // the producer warp's 32 copy arrivals and its 32 arrivals once
-            // hB is written
-            mbar_init(&full[b], 64);
+            // the producer warp's 32 copy arrivals and the arrive that counts
+            // the TMA bytes
+            mbar_init(&full[b], 33);
             mbar_init(&empty[b], ncw);
-            mbar_init(&wfull[b], 1);
         }
         unit_next = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     {
         float2 *zr = reinterpret_cast<float2 *>(smem + a.zoff);
-        for (int e = tid; e < (2 * Z + 3) * kPB; e += blockDim.x) zr[e] = make_float2(0.f, 0.f);
+        for (int e = tid; e < (2 * Z + 3) * PB; e += blockDim.x) zr[e] = make_float2(0.f, 0.f);
     }
     __syncthreads();
 
     if (warp == ncw) {
         // producer warp: the copies of item `it` go to buffer it & 1 once the
         // compute warps have released its previous use (item it - 2).  X (the
-        // box's nt x Z rows of 32 bytes) by cp.async from all 32 lanes: a
+        // box's nt x Z rows of PB x 8 bytes) by cp.async from all 32 lanes: a
         // tensor copy moves a box row per ~5 SM cycles, which rows this short
         // would make the bound; the kernel rows (2Z - 1 + kA rows) by TMA.
         int grp, own0, box0;
@@ -190,11 +219,16 @@ k_zth_apply(float2 *__restrict__ S, const __grid_constant__ CUtensorMap wmapA, c
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             unsigned char *b = smem + (size_t)buf * a.bufstride;
             zth_item(a, item, grp, own0, box0);
-            if (lane == 0) item_of[buf] = make_int3(grp, own0, box0);  // published by the arrives below
-            const int p0 = grp * kPB;
+            const int p0 = grp * PB;
+            if (lane == 0) {
+                item_of[buf] = make_int3(grp, own0, box0);  // published by the arrives below
+                mbar_expect_tx(&full[buf], a.wbytesA + a.wbytesB);
+                tma_load_2d(b + a.woff, &wmapA, p0, a.Zp - kb, &full[buf]);
+                tma_load_2d(b + a.woff + a.wbytesA, &wmapB, p0, 0, &full[buf]);
+            }
             const int nchunk = kLPR * Z * a.ntc;  // 16-byte pieces of the box's rows
-            // a piece past the plane (the last group of a plane of 2 mod 4
-            // frequencies) is not copied: its results are not stored
+            // a piece past the plane (the last group of a plane that is no
+            // multiple of PB frequencies) is not copied: its results are not stored
             const long long pc = p0 + 2 * (lane % kLPR);
             if (pc < a.plane) {
                 for (int k = lane; k < nchunk; k += 32) {
@@ -203,32 +237,13 @@ k_zth_apply(float2 *__restrict__ S, const __grid_constant__ CUtensorMap wmapA, c
                 }
             }
             cp_async_arrive(&full[buf]);
-            if (lane == 0) {
-                mbar_expect_tx(&wfull[buf], a.wbytesA + a.wbytesB);
-                tma_load_2d(b + a.woff, &wmapA, p0, a.Zp - kb, &wfull[buf]);
-                tma_load_2d(b + a.woff + a.wbytesA, &wmapB, p0, 0, &wfull[buf]);
-            }
-            // hB[s] = w[s] + w[s - 2Z + 2], s < 2Z - 1, after the kernel rows
-            if (!__all_sync(0xffffffffu, mbar_wait(&wfull[buf], (it >> 1) & 1))) {
-                if (lane == 0) atomicOr(a.err, 4u);
-                break;
-            }
-            {
-                const float2 *w = reinterpret_cast<const float2 *>(b + a.woff);
-                float2 *hbr = reinterpret_cast<float2 *>(b + a.woff + a.wbytesA + a.wbytesB);
-                for (int e = lane; e < (2 * Z - 1) * kPB; e += 32) {
-                    const int sr = e / kPB, pp = e - sr * kPB;
-                    hbr[e] = cadd(w[(sr + kb) * kPB + pp], w[(sr + ko) * kPB + pp]);
-                }
-            }
-            mbar_arrive(&full[buf]);
         }
         // no copy may still be landing when the CTA exits
         asm volatile("cp.async.wait_all;" ::: "memory");
         return;
     }
 
-    // An item's threads (kPB x Z/kTI x ntg) come in ncw warp units: unit u
+    // An item's threads (PB x nig x ntg) come in ncw warp units: unit u
     // is threads 32u .. 32u + 31 of the item.  The compute warps take the
     // units in order from a shared counter, so a warp on a less loaded SM
     // sub-partition takes more of them (ncw warps of two CTAs do not divide
@@ -252,62 +267,111 @@ k_zth_apply(float2 *__restrict__ S, const __grid_constant__ CUtensorMap wmapA, c
             return;
         }
         const int vt = unit * 32 + lane;
-        const int p = vt % kPB;
-        const int r = vt / kPB;
+        const int p = vt % PB;
+        const int r = vt / PB;
         const int ig = r % nig, tg = r / nig;
-        const int i0 = ig * kTI, tl0 = tg * kTT;  // first row, first tile of the chunk's box
+        const int i0 = ig * kTI, tl0 = tg * TT;  // first row, first tile of the chunk's box
         const float2 *X = reinterpret_cast<const float2 *>(smem + (size_t)buf * a.bufstride);
-        const float2 *W = reinterpret_cast<const float2 *>(smem + (size_t)buf * a.bufstride + a.woff);
+        const float2 *W = reinterpret_cast<const float2 *>(smem + (size_t)buf * a.bufstride + a.woff) + p;
         if (tg < a.ntg) {
-            float2 acc[kTI][kTT];
-#pragma unroll
-            for (int u = 0; u < kTI; ++u)
-#pragma unroll
-                for (int b = 0; b < kTT; ++b) acc[u][b] = make_float2(0.f, 0.f);
+            ZthAcc<TT> acc;
+            acc.clear();
             // rings: the direct value of position q (= row - column) in slot
-            // q mod 5; the reflected value of position q (= row + column), from
-            // the source of the column's class, in slot q mod 5 (i0 and the
-            // column blocks are multiples of 5).  A column that starts a
-            // segment of another class reloads the reflected ring.
-            const int wrows = a.kA + 2 * Z - 1;
-            const int zrow = (int)((a.zoff - (unsigned)buf * a.bufstride - a.woff) / (kPB * sizeof(float2)));
-            auto seg_row = [&](int k) {
-                const int cls = a.segc[k];
-                return cls == 0 ? kb : cls == 1 ? ko : cls == 2 ? wrows : zrow;
-            };
-            int sk = 0, hrow = seg_row(0), jnext = a.nseg > 1 ? a.segj[1] : Z;
+            // q mod 5; the reflected value of position q (= row + column), the
+            // sum of the sources of the column's class (the zero rows stand for
+            // an absent one), in slot q mod 5 (i0 and the column blocks are
+            // multiples of 5).  A column that starts a segment of another class
+            // reloads the reflected ring.
+            const int zrow = (int)((a.zoff - (unsigned)buf * a.bufstride - a.woff) / (PB * sizeof(float2)));
+            int sk = 0, ra = (a.segc[0] & 1) ? kb : zrow, rb = (a.segc[0] & 2) ? ko : zrow;
+            int jnext = a.nseg > 1 ? a.segj[1] : Z;
             float2 rT[kTI], rH[kTI];
 #pragma unroll
-            for (int q = 1; q < kTI; ++q) rT[q] = W[(i0 + q + kb) * kPB + p];
+            for (int q = 1; q < kTI; ++q) rT[q] = W[(i0 + q + kb) * PB];
 #pragma unroll
-            for (int q = 0; q < kTI - 1; ++q) rH[q] = W[(i0 + q + hrow) * kPB + p];
+            for (int q = 0; q < kTI - 1; ++q) rH[q] = __fadd2_rn(W[(i0 + q + ra) * PB], W[(i0 + q + rb) * PB]);
             rT[0] = rH[kTI - 1] = make_float2(0.f, 0.f);
             // the box's tiles past ntc read stale buffer contents; their
             // results are not stored
-            const float2 *xr = X + ((size_t)tl0 * Z) * kPB + p;
+            const float2 *xr = X + ((size_t)tl0 * Z) * PB + p;
             for (int j0 = 0; j0 < Z; j0 += kTI) {
+                if (ZC == 0 && j0 + kTI <= min(jnext, Z)) {
+                    // five columns of one class: no test between them, so
+                    // their loads run ahead of the products (nt = 6: 0.84
+                    // against 0.90 ms; five tiles a thread have no registers
+                    // to spare for it, and ZC > 0 tests in the columns)
 #pragma unroll
-                for (int u = 0; u < kTI; ++u) {
-                    const int j = j0 + u;
-                    rT[(kTI - u) % kTI] = W[(i0 - j + kb) * kPB + p];
-                    if (j == jnext) {
-                        ++sk;
-                        hrow = seg_row(sk);
-                        jnext = sk + 1 < a.nseg ? a.segj[sk + 1] : Z;
+                    for (int u = 0; u < kTI; ++u) {
+                        const int j = j0 + u;
+                        rT[(kTI - u) % kTI] = W[(i0 - j + kb) * PB];
+                        rH[(u + kTI - 1) % kTI] =
+                            __fadd2_rn(W[(i0 + j + kTI - 1 + ra) * PB], W[(i0 + j + kTI - 1 + rb) * PB]);
+                        float2 m[kTI], x[TT];
 #pragma unroll
-                        for (int q = 0; q < kTI - 1; ++q) rH[(q + u) % kTI] = W[(i0 + j + q + hrow) * kPB + p];
+                        for (int q = 0; q < kTI; ++q)
+                            m[q] = __fadd2_rn(rT[(q - u + kTI) % kTI], rH[(q + u) % kTI]);
+#pragma unroll
+                        for (int b = 0; b < TT; ++b) x[b] = xr[((size_t)b * Z + j) * PB];
+                        acc.add(m, x);
                     }
-                    rH[(u + kTI - 1) % kTI] = W[(i0 + j + kTI - 1 + hrow) * kPB + p];
-                    float2 m[kTI];
+                    continue;
+                }
+                if constexpr (ZC > 0) {
+                    static_assert(ZC % kTI == 0, "a depth of whole column blocks");
 #pragma unroll
-                    for (int q = 0; q < kTI; ++q) m[q] = cadd(rT[(q - u + kTI) % kTI], rH[(q + u) % kTI]);
-                    float2 x[kTT];
+                    for (int u = 0; u < kTI; ++u) {
+                        const int j = j0 + u;
+                        rT[(kTI - u) % kTI] = W[(i0 - j + kb) * PB];
+                        if (j == jnext) {
+                            ++sk;
+                            ra = (a.segc[sk] & 1) ? kb : zrow;
+                            rb = (a.segc[sk] & 2) ? ko : zrow;
+                            jnext = sk + 1 < a.nseg ? a.segj[sk + 1] : Z;
 #pragma unroll
-                    for (int b = 0; b < kTT; ++b) x[b] = xr[((size_t)b * Z + j) * kPB];
+                            for (int q = 0; q < kTI - 1; ++q)
+                                rH[(q + u) % kTI] = __fadd2_rn(W[(i0 + j + q + ra) * PB], W[(i0 + j + q + rb) * PB]);
+                        }
+                        rH[(u + kTI - 1) % kTI] =
+                            __fadd2_rn(W[(i0 + j + kTI - 1 + ra) * PB], W[(i0 + j + kTI - 1 + rb) * PB]);
+                        float2 m[kTI], x[TT];
 #pragma unroll
-                    for (int q = 0; q < kTI; ++q)
+                        for (int q = 0; q < kTI; ++q) m[q] = __fadd2_rn(rT[(q - u + kTI) % kTI], rH[(q + u) % kTI]);
 #pragma unroll
-                        for (int b = 0; b < kTT; ++b) acc[q][b] = cfma(m[q], x[b], acc[q][b]);
+                        for (int b = 0; b < TT; ++b) x[b] = xr[((size_t)b * Z + j) * PB];
+                        acc.add(m, x);
+                    }
+                } else {
+                    // a block with a change of class, or cut at Z: one column
+                    // at a time, the rings turned by a place after each
+                    const int n = min(kTI, Z - j0);
+#pragma unroll 1
+                    for (int u = 0; u < n; ++u) {
+                        const int j = j0 + u;
+                        rT[0] = W[(i0 - j + kb) * PB];
+                        if (j == jnext) {
+                            ++sk;
+                            ra = (a.segc[sk] & 1) ? kb : zrow;
+                            rb = (a.segc[sk] & 2) ? ko : zrow;
+                            jnext = sk + 1 < a.nseg ? a.segj[sk + 1] : Z;
+#pragma unroll
+                            for (int q = 0; q < kTI - 1; ++q)
+                                rH[q] = __fadd2_rn(W[(i0 + j + q + ra) * PB], W[(i0 + j + q + rb) * PB]);
+                        }
+                        rH[kTI - 1] = __fadd2_rn(W[(i0 + j + kTI - 1 + ra) * PB], W[(i0 + j + kTI - 1 + rb) * PB]);
+                        float2 m[kTI], x[TT];
+#pragma unroll
+                        for (int q = 0; q < kTI; ++q) m[q] = __fadd2_rn(rT[q], rH[q]);
+#pragma unroll
+                        for (int b = 0; b < TT; ++b) x[b] = xr[((size_t)b * Z + j) * PB];
+                        acc.add(m, x);
+                        const float2 t4 = rT[kTI - 1], h0 = rH[0];
+#pragma unroll
+                        for (int q = kTI - 1; q > 0; --q) rT[q] = rT[q - 1];
+#pragma unroll
+                        for (int q = 0; q < kTI - 1; ++q) rH[q] = rH[q + 1];
+                        rT[0] = t4;
+                        rH[kTI - 1] = h0;
+                    }
                 }
             }
             // the operands are in registers: release the buffer before the stores
@@ -315,18 +379,19 @@ k_zth_apply(float2 *__restrict__ S, const __grid_constant__ CUtensorMap wmapA, c
             const int own0 = ii.y, box0 = ii.z;
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[buf]);
-            const long long pg = (long long)ii.x * kPB + p;
+            const long long pg = (long long)ii.x * PB + p;
             if (pg < a.plane) {
                 const float f = a.fresp ? a.fresp[pg] : 1.f;
                 // box0 + ntc >= t_end: the condition keeps t inside the box
                 const int t_end = CH ? min(own0 + a.ntc, a.nt) : a.nt;
 #pragma unroll
-                for (int b = 0; b < kTT; ++b) {
+                for (int b = 0; b < TT; ++b) {
                     const int t = CH ? box0 + tl0 + b : tl0 + b;
                     if ((!CH || t >= own0) && t < t_end) {
 #pragma unroll
                         for (int q = 0; q < kTI; ++q)
-                            S[((long long)t * Z + i0 + q) * a.plane + pg] = cscale(acc[q][b], f);
+                            if (ZC > 0 || i0 + q < Z)
+                                S[((long long)t * Z + i0 + q) * a.plane + pg] = cscale(acc.get(q, b), f);
                     }
                 }
             }
@@ -369,9 +434,9 @@ int make_map(CUtensorMap *m, const void *base, int rank, const cuuint64_t *dims,
     return MM_OK;
 }
 
-// the compute warps (threads kPB x Z/kTI x ntg, rounded up to whole warps)
-// and the producer warp
-int zth_threads(int Z, int ntg) { return ((kPB * (Z / kTI) * ntg + 31) / 32 + 1) * 32; }
+// the compute warps (threads PB x ceil(Z / kTI) x ntg, rounded up to whole
+// warps) and the producer warp
+int zth_threads(int Z, int pb, int ntg) { return ((pb * ((Z + kTI - 1) / kTI) * ntg + 31) / 32 + 1) * 32; }
 
 // staged row of w[0]: the rows -(2Z-2) .. -1 rounded up to a multiple of four,
 // so that the second kernel box starts on a 128-byte boundary
@@ -379,44 +444,85 @@ int zth_ka(int Z) { return (2 * Z - 2 + 3) & ~3; }
 
 // bytes per buffer: X for ntg whole tile groups (the last group's threads
 // read tiles past the box, whose results are not stored), then the kernel
-// rows -kA .. 2Z - 2 and hB[0 .. 2Z - 2]; both parts start on 128-byte
-// boundaries
-size_t zth_bufstride(int Z, int ntg, unsigned *woff) {
-    const size_t xb = (size_t)kPB * Z * ntg * kTT * sizeof(float2);
-    const size_t wb = (size_t)kPB * (zth_ka(Z) + 2 * Z - 1 + 2 * Z - 1) * sizeof(float2);
+// rows -kA .. 2Z - 2 and four more that the cut row group of a depth that is no
+// multiple of kTI reads for rows it does not store; both parts start on
+// 128-byte boundaries
+size_t zth_bufstride(int Z, int pb, int tiles, unsigned *woff) {
+    const size_t xb = (size_t)pb * Z * tiles * sizeof(float2);
+    const size_t wb = (size_t)pb * (zth_ka(Z) + 2 * Z - 1 + 4) * sizeof(float2);
     const size_t xo = (xb + 127) & ~(size_t)127;
     if (woff) *woff = (unsigned)xo;
     return (xo + wb + 127) & ~(size_t)127;
 }
 
-// shared memory of one CTA, two CTAs per SM
-constexpr size_t kSmemMax = 112 * 1024;
+// shared memory of an SM's CTAs
+constexpr size_t kSmemMax = 224 * 1024;
 
 // the zero rows after the two buffers
-size_t zth_zero_bytes(int Z) { return ((size_t)(2 * Z + 3) * kPB * sizeof(float2) + 127) & ~(size_t)127; }
+size_t zth_zero_bytes(int Z, int pb) { return ((size_t)(2 * Z + 3) * pb * sizeof(float2) + 127) & ~(size_t)127; }
 
-// How a batch of nt tiles is split: the fewest chunks whose tile groups fit
-// one CTA (threads and shared memory), then the tiles spread evenly over them.
+// How a batch of nt tiles runs: TT tiles per thread, PB frequencies per group,
+// and the fewest chunks whose tile groups fit one CTA (threads and shared
+// memory), the tiles spread evenly over them.
 struct ZthPlan {
-    int nchunks, ntc, ntg;
+    int tt, pb, nchunks, ntc, ntg;
 };
-bool zth_plan(int Z, int nt, ZthPlan *pl) {
-    const int ntg_all = (nt + kTT - 1) / kTT;
+bool zth_fits(int Z, int pb, int tt, int ntg) {
+    return zth_threads(Z, pb, ntg) <= zth_max_threads(tt, pb) &&
+           2 * zth_bufstride(Z, pb, ntg * tt, nullptr) + zth_zero_bytes(Z, pb) <= kSmemMax / zth_ctas(tt, pb);
+}
+bool zth_split(int Z, int nt, int tt, int pb, ZthPlan *pl) {
+    const int ntg_all = (nt + tt - 1) / tt;
     int ntg_max = ntg_all;
-    while (ntg_max > 0 && (zth_threads(Z, ntg_max) > kThreadsMax ||
-                           2 * zth_bufstride(Z, ntg_max, nullptr) + zth_zero_bytes(Z) > kSmemMax))
-        --ntg_max;
+    while (ntg_max > 0 && !zth_fits(Z, pb, tt, ntg_max)) --ntg_max;
     if (ntg_max == 0) return false;
+    pl->tt = tt;
+    pl->pb = pb;
     pl->nchunks = (ntg_all + ntg_max - 1) / ntg_max;
     pl->ntc = (nt + pl->nchunks - 1) / pl->nchunks;
-    pl->ntg = (pl->ntc + kTT - 1) / kTT;
+    pl->ntg = (pl->ntc + tt - 1) / tt;
     return true;
+}
+// Measured at P = 678 (ms per launch; the per-tile form, or for Z = 37 the
+// direct sum, in brackets): Z = 50, 2 tiles, 16 frequencies of 2 tiles a thread
+// 0.32 [0.40]; 3 tiles, 8 x 3 0.50 [0.56]; 4 tiles, 8 x 2 0.59, 8 x 5 0.67
+// [0.75]; 6 tiles, 8 x 3 0.80, 8 x 5 1.06 [1.12]; 9 tiles, 8 x 5 1.12, 8 x 3
+// 1.25, 4 x 5 1.20 [2.27 at zpad 24]; 16 tiles, 4 x 5 2.06, 8 x 5 2.11; 25
+// tiles, 4 x 5 2.69, 8 x 5 2.75; Z = 37, 9 tiles, 8 x 5 0.70 [2.14], 25 tiles,
+// 8 x 5 1.78, 4 x 5 2.06.  So few tiles take as many per thread as leave no
+// place empty and wide groups (a row of 8 frequencies is 64 bytes); from 11
+// tiles on the groups are narrow for a depth of whole row groups, where two CTAs
+// share an SM, and wide for a cut one while a single chunk fits.
+bool zth_plan(int Z, int nt, ZthPlan *pl) {
+#ifdef ZTH_FORCE
+    return zth_split(Z, nt, g_tt, g_pb, pl);
+#endif
+    if (nt <= 10) {
+        const int tt = nt <= 3 ? nt : nt == 4 ? 2 : nt == 6 ? 3 : 5;
+        if (zth_split(Z, nt, tt, nt <= 2 ? 16 : 8, pl) && pl->nchunks == 1) return true;
+    } else if (Z % kTI != 0) {
+        if (zth_split(Z, nt, 5, 8, pl) && pl->nchunks == 1) return true;
+    }
+    return zth_split(Z, nt, 5, 4, pl);
+}
+
+const void *zth_kernel(int Z, const ZthPlan &pl) {
+    if (pl.nchunks > 1) return (const void *)k_zth_apply<0, 5, 4, true>;
+    switch (pl.tt * 100 + pl.pb) {
+        case 504: return Z == 50 ? (const void *)k_zth_apply<50, 5, 4, false> : (const void *)k_zth_apply<0, 5, 4, false>;
+        case 508: return (const void *)k_zth_apply<0, 5, 8, false>;
+        case 308: return (const void *)k_zth_apply<0, 3, 8, false>;
+        case 208: return (const void *)k_zth_apply<0, 2, 8, false>;
+        case 216: return (const void *)k_zth_apply<0, 2, 16, false>;
+        case 116: return (const void *)k_zth_apply<0, 1, 16, false>;
+    }
+    return nullptr;
 }
 
 }  // namespace
 
 int mm_zth_supported(int Z, int zpad, int nt, long long plane) {
-    if (Z < kTI || Z % kTI != 0 || zpad < 1 || zpad > Z - 1 || nt < 1 || plane % 2 != 0) return 0;
+    if (Z < 2 || zpad < 1 || zpad > Z - 1 || nt < 1 || plane % 2 != 0) return 0;
     if (2 * Z - 1 > 256 || zth_ka(Z) > 256) return 0;  // TMA box height
     ZthPlan pl;
     return zth_plan(Z, nt, &pl) && encode_fn() != nullptr ? pl.nchunks : 0;
@@ -430,11 +536,11 @@ int mm_launch_zth_apply(float2 *S, const float2 *w, int Z, int zpad, int Zp, lon
     ZthPlan pl;
     zth_plan(Z, nt, &pl);
     CUtensorMap wA, wB;
-    const cuuint32_t kb = (cuuint32_t)(2 * Z - 2), kA = (cuuint32_t)zth_ka(Z);
+    const cuuint32_t kb = (cuuint32_t)(2 * Z - 2), kA = (cuuint32_t)zth_ka(Z), pb = (cuuint32_t)pl.pb;
     {
         cuuint64_t dims[2] = {(cuuint64_t)plane, (cuuint64_t)Zp};
         cuuint64_t strides[1] = {(cuuint64_t)plane * 8};
-        cuuint32_t boxA[2] = {kPB, kA}, boxB[2] = {kPB, kb + 1};
+        cuuint32_t boxA[2] = {pb, kA}, boxB[2] = {pb, kb + 1};
         if (int rc = make_map(&wA, w, 2, dims, strides, boxA)) return rc;
         if (int rc = make_map(&wB, w, 2, dims, strides, boxB)) return rc;
     }
@@ -446,14 +552,14 @@ int mm_launch_zth_apply(float2 *S, const float2 *w, int Z, int zpad, int Zp, lon
     a.ntg = pl.ntg;
     a.nchunks = pl.nchunks;
     a.plane = plane;
-    const long long nitems = ((plane + kPB - 1) / kPB) * pl.nchunks;
+    const long long nitems = ((plane + pl.pb - 1) / pl.pb) * pl.nchunks;
     MM_REQUIRE(nitems < (1LL << 31), "z operator: too many frequency groups");
     a.nitems = (int)nitems;
     // the column segments of one reflection class
     a.nseg = 0;
     for (int j = 0, prev = -1; j < Z; ++j) {
         const bool vin = j >= 1 && j <= zpad, vout = j >= Z - 1 - zpad && j <= Z - 2;
-        const int cls = vin ? (vout ? 2 : 0) : (vout ? 1 : 3);
+        const int cls = (vin ? 1 : 0) | (vout ? 2 : 0);
         if (cls != prev) {
             MM_REQUIRE(a.nseg < 6, "z operator: more than six column segments");
             a.segj[a.nseg] = j;
@@ -463,21 +569,19 @@ int mm_launch_zth_apply(float2 *S, const float2 *w, int Z, int zpad, int Zp, lon
         }
     }
     a.kA = (int)kA;
-    a.xbytes = (unsigned)(kPB * Z * pl.ntc * sizeof(float2));
-    a.wbytesA = (unsigned)(kPB * kA * sizeof(float2));
-    a.wbytesB = (unsigned)(kPB * (kb + 1) * sizeof(float2));
-    a.bufstride = (unsigned)zth_bufstride(Z, pl.ntg, &a.woff);
+    a.wbytesA = (unsigned)(pl.pb * kA * sizeof(float2));
+    a.wbytesB = (unsigned)(pl.pb * (kb + 1) * sizeof(float2));
+    a.bufstride = (unsigned)zth_bufstride(Z, pl.pb, pl.ntg * pl.tt, &a.woff);
     a.zoff = 2 * a.bufstride;
     MM_REQUIRE(a.bufstride % 128 == 0 && a.woff % 128 == 0 && a.wbytesA % 128 == 0,
                "TMA destinations of the z operator must be 128-byte aligned");
-    MM_REQUIRE(a.xbytes <= a.woff, "z operator: the X box overruns its buffer");
+    MM_REQUIRE((size_t)pl.pb * Z * pl.ntc * sizeof(float2) <= a.woff, "z operator: the X box overruns its buffer");
     a.fresp = fresp;
     a.err = err;
-    const size_t sm = 2 * (size_t)a.bufstride + zth_zero_bytes(Z);
-    const int threads = zth_threads(Z, a.ntg);
-    const void *fn = pl.nchunks > 1 ? (const void *)k_zth_apply<0, true>
-                     : Z == 50     ? (const void *)k_zth_apply<50, false>
-                                   : (const void *)k_zth_apply<0, false>;
+    const size_t sm = 2 * (size_t)a.bufstride + zth_zero_bytes(Z, pl.pb);
+    const int threads = zth_threads(Z, pl.pb, a.ntg);
+    const void *fn = zth_kernel(Z, pl);
+    MM_REQUIRE(fn != nullptr, "z operator: no kernel for %d tiles per thread, %d frequencies", pl.tt, pl.pb);
     if (int rc = mm_set_smem(fn, sm)) return rc;
     int per_sm = 0;
     MM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, sm));

@@ -489,6 +489,61 @@ def test_per_tile_z_operator_full_variant_restates_the_matrix(Z):
     np.testing.assert_allclose(got, M, rtol=0, atol=1e-12)
 
 
+def test_z_operator_rings_at_any_depth():
+    """k_zth_apply (csrc/zop_tma.cu) at depths that are no multiple of its five
+    rows, and at those that are: the reflected ring is the sum of the kernel
+    rows at the offsets of the column's class, the zero rows standing for an
+    absent reflection; the last row group and column block are cut.  Against M
+    built from the padding map, every read inside the staged rows (kA + 2Z - 1
+    and four more) or the 2Z + 3 zero rows."""
+    rng = np.random.default_rng(6)
+    for Z, zpad in [(2, 1), (3, 2), (3, 1), (4, 3), (7, 2), (12, 11), (37, 36), (37, 18), (41, 40), (50, 49), (50, 24),
+                    (64, 5), (80, 79), (123, 122)]:
+        Zp = Z + 2 * zpad
+        w = rng.standard_normal(Zp) + 1j * rng.standard_normal(Zp)
+        M = np.zeros((Z, Z), complex)
+        for z in range(Zp):
+            j = int(_map_z(z, Z, zpad, Zp))
+            if j >= 0:
+                for i in range(Z):
+                    M[i, j] += w[(zpad + i - z) % Zp]
+        kb = (2 * Z - 2 + 3) & ~3
+        ko = kb - (2 * Z - 2)
+        staged = np.full(kb + 2 * Z - 1 + 4, np.nan, complex)  # the four rows past the boxes hold anything
+        for row in range(kb + 2 * Z - 1):
+            src = Zp - kb + row if row < kb else row - kb
+            staged[row] = w[src] if 0 <= src < Zp else 0
+        zrow, zeros = 10000, np.zeros(2 * Z + 3, complex)
+        cls = [(1 if 1 <= j <= zpad else 0) | (2 if Z - 1 - zpad <= j <= Z - 2 else 0) for j in range(Z)]
+        segj = [j for j in range(Z) if j == 0 or cls[j] != cls[j - 1]]
+        assert len(segj) <= 6
+
+        def at(i):
+            if i >= zrow:
+                assert i - zrow < len(zeros), i
+                return zeros[i - zrow]
+            assert 0 <= i < len(staged), i
+            return staged[i]
+
+        got = np.zeros((Z, Z), complex)
+        for i0 in range(0, Z, 5):
+            def two(i, j):
+                return at(i + (kb if cls[j] & 1 else zrow)) + at(i + (ko if cls[j] & 2 else zrow))
+            rT = [0j] + [at(i0 + q + kb) for q in range(1, 5)]
+            rH = [two(i0 + q, 0) for q in range(4)] + [0j]
+            for j in range(Z):
+                u = j % 5
+                rT[(5 - u) % 5] = at(i0 - j + kb)
+                if j in segj[1:]:
+                    for q in range(4):
+                        rH[(q + u) % 5] = two(i0 + j + q, j)
+                rH[(u + 4) % 5] = two(i0 + j + 4, j)
+                for q in range(5):
+                    if i0 + q < Z:
+                        got[i0 + q, j] = rT[(q - u + 5) % 5] + rH[(q + u) % 5]
+        np.testing.assert_allclose(got, M, rtol=0, atol=1e-12)
+
+
 def _unit_protocol_run(rng, nwarps, nunits, nitems):
     """One simulated run of the register z operator's warp-unit protocol
     (csrc/zop_tma.cu): nwarps compute warps take units in order from a shared
