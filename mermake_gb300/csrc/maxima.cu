@@ -281,7 +281,11 @@ k_maxima(Vols V, float th, int delta, Xform t, uint2 *__restrict__ cand, unsigne
     const bool skip_small = t.div > 0.f && th > 0.f;
     // the two-sign pass with th >= 0 (not NaN): one queue round per voxel
     const bool excl = both && th >= 0.f;
+    const bool skip_chunk = skip_small || (t.div == 0.f && th >= 0.f);
     const float lo = skip_small ? th * t.div * (1.f - 0x1p-18f) : 0.f;
+    const float chunk_th = skip_small ? lo : th;
+    const unsigned keep_bits = skip_small || both ? 0x7fffffffu : 0xffffffffu;  // |value|, or value
+    const unsigned flip_bits = !(skip_small || both) && t.neg ? 0x80000000u : 0u;
     unsigned *my_k = qk[warp];
     int *my_y = qy[warp];
     float *my_v = qv[warp];
@@ -297,6 +301,19 @@ k_maxima(Vols V, float th, int delta, Xform t, uint2 *__restrict__ cand, unsigne
             for (int k = 0; k < kMaxY; ++k) {
                 const int y = y0 + 32 * k + (int)lane;
                 vals[k] = y < yhi ? rp[y] : 0.f;
+            }
+            // a chunk without a value the threshold lets pass (most chunks of a
+            // volume thresholded above its noise) ends here.  With a divisor the
+            // test is the one that spares the quotient; without one the value
+            // itself is compared, in the sign asked for (a NaN passes).  DAPI
+            // block of 50 x 1500 x 1302: 0.74 -> 0.61 ms with its fits,
+            // a colour of 25 tiles 0.36 -> 0.24
+            if (skip_chunk) {
+                bool some = false;
+#pragma unroll
+                for (int k = 0; k < kMaxY; ++k)
+                    some |= !(__uint_as_float((__float_as_uint(vals[k]) & keep_bits) ^ flip_bits) <= chunk_th);
+                if (!__any_sync(0xffffffffu, some)) continue;
             }
             // queue the voxels above the threshold (maxima.cu:19; a NaN
             // threshold admits every voxel) whose y neighbours held by the

@@ -244,6 +244,48 @@ def test_reflect_errors(mm):
     assert r(a, i=1, out=out) is out
 
 
+@pytest.mark.parametrize("shape", [(3, 5, 64), (2, 7, 65), (1, 3, 515), (4, 130), (2050,), (2, 3, 600)])
+@pytest.mark.parametrize("cut", [(0, 0), (1, 0), (0, 1), (3, 2)])
+def test_subtract_u16_dense_rows(mm, shape, cut):
+    """Rows that start on either half of a word in each of the three arrays
+    (views cut by `cut` pixels), odd lengths, one to three axes, and an array
+    that is its own result."""
+    rng = np.random.default_rng(sum(shape))
+    a, b = (rng.integers(0, 65536, shape[:-1] + (shape[-1] + 5,)).astype(np.uint16) for _ in range(2))
+    n = shape[-1]
+    dev = [torch.from_numpy(v.view(np.int16)).cuda().view(torch.uint16) for v in (a, b)]
+    va, vb = dev[0][..., cut[0]:cut[0] + n], dev[1][..., cut[1]:cut[1] + n]
+    ia, ib = a[..., cut[0]:cut[0] + n].astype(np.int64), b[..., cut[1]:cut[1] + n].astype(np.int64)
+    for fn, want in ((mm["math"].subtract_reflect, np.abs(ia - ib)), (mm["math"].subtract_clamp, np.maximum(ia - ib, 0))):
+        got = fn(va, vb).view(torch.int16).cpu().numpy().view(np.uint16)
+        np.testing.assert_array_equal(got, want)
+    mm["math"].subtract_clamp(va, vb, out=va)
+    full = dev[0].view(torch.int16).cpu().numpy().view(np.uint16)
+    a[..., cut[0]:cut[0] + n] = np.maximum(ia - ib, 0)
+    np.testing.assert_array_equal(full, a)
+
+
+@pytest.mark.parametrize("neg,div,th", [(False, 0.0, 0.0), (True, 0.0, 40.0), (False, 2.5, 30.0), (True, 2.5, 0.0),
+                                        (False, 0.0, -5.0)])
+def test_maxima_chunks_without_a_candidate(mm, neg, div, th):
+    """Rows of several scan chunks of which most hold no value above the
+    threshold, a NaN among them: the same maxima as the oracle's."""
+    rng = np.random.default_rng(17)
+    im = rng.normal(0, 1, (5, 9, 700)).astype(np.float32)
+    at = tuple(rng.integers(0, n, 60) for n in im.shape)
+    im[at] += rng.choice([-1, 1], 60).astype(np.float32) * 200
+    got = mm["maxima"].find_local_maxima(torch.from_numpy(im).cuda(), th, 1, 1, norm_div=div, negate=neg).cpu().numpy()
+    v = im / np.float32(div) if div else im
+    v = -v if neg else v
+    want = ck.find_local_maxima(np.ascontiguousarray(v), th, 1, 1, im, 1.0, 1.5)
+    assert len(want) > 20
+    assert_rows_close(got, want)
+    im[2, 4, 333] = np.nan  # admitted by every threshold, and never below a neighbour
+    t = torch.from_numpy(im).cuda()
+    with_nan = mm["maxima"].find_local_maxima(t, th, 1, 0, norm_div=div, negate=neg)
+    assert bool(torch.isnan(with_nan[:, 7]).any())
+
+
 def test_subtract_u16(mm):
     rng = np.random.default_rng(2)
     x = rng.integers(0, 65536, (4, 7, 9)).astype(np.uint16)
