@@ -11,10 +11,10 @@
 // (align.py:61-77).
 //
 // The correlation of two 0/1 images at shift s is the number of voxel pairs
-// (i in moving, j in reference) with i - j = s, so it is computed exactly as a
-// histogram of pair differences instead of an FFT (whose float result rounds
-// to the same integers); the argmax takes the first maximal index in C order,
-// as argmax does.  Nearest neighbours are brute force in double precision,
+// (i in moving, j in reference) with i - j = s, so it is computed exactly by
+// counting pair differences, a row of shifts at a time in shared memory,
+// instead of an FFT (whose float result rounds to the same integers); the argmax
+// takes the first maximal index in C order, as argmax does.  Nearest neighbours are brute force in double precision,
 // ties to the lowest reference index.
 #include <limits.h>
 #include <math.h>
@@ -29,12 +29,13 @@
 // per-aligner scratch for the moving sets, grown on demand
 struct MmDriftWork {
     float *pts = nullptr;
-    int *iv = nullptr, *keep = nullptr, *small = nullptr, *vox = nullptr;
+    int *iv = nullptr, *keep = nullptr, *small = nullptr;
+    int *xs = nullptr, *ys = nullptr;  // x and y of the unique voxels, row (z, x) by row
     size_t cap = 0;
     unsigned char *grid = nullptr;
     size_t grid_bytes = 0;
-    int *hist = nullptr;
-    size_t hist_bytes = 0;
+    int *rows = nullptr;      // first voxel of each row, and their number at the end
+    size_t rows_cap = 0;
     int *h_small = nullptr;
 };
 
@@ -48,15 +49,16 @@ struct MmCellGrid {
     int *start = nullptr;     // device, cells + 1: first sorted point of each cell
     float *pts = nullptr;     // device, n x 3: points sorted by cell (index order within a cell)
     int *idx = nullptr;       // device, n: original index of each sorted point
-    double *state = nullptr;  // device: shift (3), integer-shift flag, matched count
-    double *parts = nullptr;  // device: per-block partial sums of a refinement round
+    double *state = nullptr;  // device, two slots: shift (3), integer-shift flag, matched count
+    double *parts = nullptr;  // device, two slots: per-block partial sums of a refinement round
 };
 
 struct mm_aligner {
     int n;            // reference points kept by the threshold
     float *pts;       // device, n x 3
     int nvox;         // unique reference voxels
-    int *vox;         // device, nvox x 3 (z, x, y)
+    int *rows;        // device, shape[0] x shape[1] + 1: first voxel of each (z, x) row
+    int *ys;          // device, nvox: the voxels' y
     int shape[3];     // reference image shape
     int resc, trim;
     float th;         // NaN: no threshold
@@ -148,60 +150,139 @@ __global__ void k_mark(const int *__restrict__ iv, const int *__restrict__ keep,
     }
 }
 
-// unique voxels of the grid, any order
-__global__ void k_grid_list(const unsigned char *__restrict__ grid, long long total, int s1, int s2,
-                            int *__restrict__ vox, int *__restrict__ nvox) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        if (!grid[i]) continue;
-        const int p = atomicAdd(nvox, 1);
-        vox[p * 3 + 0] = (int)(i / ((long long)s1 * s2));
-        vox[p * 3 + 1] = (int)((i / s2) % s1);
-        vox[p * 3 + 2] = (int)(i % s2);
+// The unique voxels of the grid as rows (z, x): a warp counts a row's, one CTA
+// turns the counts into starts (rows[nrows] the total), a warp lists its voxels.
+__global__ void k_row_count(const unsigned char *__restrict__ grid, int nrows, int s2, int *__restrict__ rows) {
+    const int lane = threadIdx.x & 31;
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += (gridDim.x * blockDim.x) >> 5) {
+        int c = 0;
+        for (int y = lane; y < s2; y += 32) c += grid[(long long)r * s2 + y];
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) rows[r] = c;
+    }
+}
+__global__ void __launch_bounds__(1024) k_row_scan(int *__restrict__ rows, int nrows) {
+    __shared__ int part[32];
+    __shared__ int base;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) base = 0;
+    for (int r0 = 0; r0 < nrows; r0 += 1024) {
+        const int r = r0 + threadIdx.x, c = r < nrows ? rows[r] : 0;
+        int v = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += t;
+        }
+        if (lane == 31) part[warp] = v;
+        __syncthreads();
+        if (warp == 0) {
+            int p = part[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, p, o);
+                if (lane >= o) p += t;
+            }
+            part[lane] = p;
+        }
+        __syncthreads();
+        const int before = base + (warp ? part[warp - 1] : 0) + v - c;
+        if (r < nrows) rows[r] = before;
+        __syncthreads();
+        if (threadIdx.x == 1023) base = before + c;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) rows[nrows] = base;
+}
+__global__ void k_row_fill(const unsigned char *__restrict__ grid, int nrows, int s1, int s2,
+                           const int *__restrict__ rows, int *__restrict__ xs, int *__restrict__ ys) {
+    const int lane = threadIdx.x & 31;
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrows; r += (gridDim.x * blockDim.x) >> 5) {
+        int at = rows[r];
+        if (at == rows[r + 1]) continue;
+        for (int y0 = 0; y0 < s2; y0 += 32) {
+            const bool on = y0 + lane < s2 && grid[(long long)r * s2 + y0 + lane];
+            const unsigned m = __ballot_sync(0xffffffffu, on);
+            if (on) {
+                const int v = at + __popc(m & ((1u << lane) - 1));
+                xs[v] = r % s1;
+                ys[v] = y0 + lane;
+            }
+            at += __popc(m);
+        }
     }
 }
 
-// correlation as a histogram of pair differences: output index i - j + (sb - 1)
-__global__ void k_pair_hist(const int *__restrict__ a, const int *__restrict__ na, const int *__restrict__ b,
-                            int nb, int c0, int c1, int c2, int o1, int o2, int *__restrict__ hist) {
-    const long long total = (long long)(*na) * nb;
-    for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < total;
-         p += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(p / nb), j = (int)(p % nb);
-        const int z = a[i * 3 + 0] - b[j * 3 + 0] + c0;
-        const int x = a[i * 3 + 1] - b[j * 3 + 1] + c1;
-        const int y = a[i * 3 + 2] - b[j * 3 + 2] + c2;
-        atomicAdd(&hist[((long long)z * o1 + x) * o2 + y], 1);
-    }
-}
-
-// first index of the maximum: max of (count << 32 | ~index)
-__global__ void k_argmax(const int *__restrict__ hist, long long total, unsigned long long *__restrict__ best) {
-    unsigned long long b = 0;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += (long long)gridDim.x * blockDim.x) {
-        const unsigned long long key = ((unsigned long long)(unsigned)hist[i] << 32) | (unsigned)(~(unsigned)i);
-        b = key > b ? key : b;
+// The correlation peak: a CTA takes a row (z, x) of shifts, i.e. the pairs of
+// rows (az, ax) of the moving and (az - dz, ax - dx) of the reference voxels,
+// counts their y differences in shared memory (kCorrSeg shifts at a time), and
+// offers its first largest count, as (count << 32 | ~index).  Counting in one
+// histogram of all shifts in global memory took 141 us for 6000 x 6000 voxels
+// (36 M additions in L2), clearing and searching it 40 us more.
+constexpr int kCorrThreads = 64, kCorrSeg = 1024;
+struct CorrShape {
+    int a[2], b[2];  // rows of the two sets: (z, x) extents
+    int o1, o2;      // extents of the shifts along x and y
+    int c2;          // y shift of index 0 (negated)
+    long long nout;  // rows of shifts
+};
+__global__ void __launch_bounds__(kCorrThreads)
+k_corr_rows(const int *__restrict__ ra, const int *__restrict__ xa, const int *__restrict__ ya,
+            const int *__restrict__ rb, const int *__restrict__ yb, CorrShape s, unsigned long long *__restrict__ best) {
+    __shared__ int hist[kCorrSeg];
+    unsigned long long mine = 0;
+    for (long long out = blockIdx.x; out < s.nout; out += gridDim.x) {
+        const int oz = (int)(out / s.o1), ox = (int)(out - (long long)oz * s.o1);
+        const int dz = oz - (s.b[0] - 1), dx = ox - (s.b[1] - 1);
+        const int z0 = max(0, dz), z1 = min(s.a[0], s.b[0] + dz), x0 = max(0, dx), x1 = min(s.a[1], s.b[1] + dx);
+        for (int y0 = 0; y0 < s.o2; y0 += kCorrSeg) {
+            const int ny = min(kCorrSeg, s.o2 - y0);
+            for (int y = threadIdx.x; y < ny; y += kCorrThreads) hist[y] = 0;
+            __syncthreads();
+            // the moving voxels of rows (z, x0 .. x1) are consecutive: a thread
+            // each, against the voxels of its reference row
+            if (ra && x0 < x1)
+                for (int z = z0; z < z1; ++z) {
+                    const int p1 = ra[z * s.a[1] + x1], jrow = (z - dz) * s.b[1] - dx;
+                    for (int p = ra[z * s.a[1] + x0] + threadIdx.x; p < p1; p += kCorrThreads) {
+                        const int j = jrow + xa[p], q1 = rb[j + 1], y = ya[p] + s.c2 - y0;
+                        for (int q = rb[j]; q < q1; ++q) {
+                            const int d = y - yb[q];
+                            if ((unsigned)d < (unsigned)ny) atomicAdd(&hist[d], 1);
+                        }
+                    }
+                }
+            __syncthreads();
+            const long long at = out * s.o2 + y0;
+            for (int y = threadIdx.x; y < ny; y += kCorrThreads) {
+                const unsigned long long key = ((unsigned long long)(unsigned)hist[y] << 32) | (unsigned)~(unsigned)(at + y);
+                mine = key > mine ? key : mine;
+            }
+            __syncthreads();
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long t = __shfl_xor_sync(0xffffffffu, b, o);
-        b = t > b ? t : b;
+        const unsigned long long t = __shfl_xor_sync(0xffffffffu, mine, o);
+        mine = t > mine ? t : mine;
     }
-    if ((threadIdx.x & 31) == 0) atomicMax(best, b);
+    if ((threadIdx.x & 31) == 0) atomicMax(best, mine);
 }
 
-// five nearest-neighbour refinements in one CTA (align.py:61-77).  t0: the
-// coarse shift (integer, times resc).  out: tzxy (3 floats) and the count of
-// the last round.
 // Nearest-neighbour refinement (align.py:55-76, five rounds with radii
 // np.linspace(resc, target, 5)), one round per launch over many CTAs.  Each
 // moving point X - shift looks for its nearest reference point among the
-// cells around it (distance in double, ties to the lower reference index:
-// the point a brute-force search over all references would pick); if it lies
-// within the round's radius, X - R (float32) is added in double.  Blocks
-// write partial sums that k_refine_update adds in a fixed order.
+// cells that its match radius reaches (distance in double, ties to the lower
+// reference index: the point a brute-force search over all references would
+// pick); if it lies within the round's radius, X - R (float32) is added in
+// double.  Eight lanes share a point's rows of cells, since a search is a chain
+// of dependent loads, and the cells are found in float, the reach widened by
+// more than its rounding, since this part does two double products per SM and
+// cycle (a thread per point with double quotients: 22 us a round for 6000
+// points).  Blocks write partial sums, which every block of the next round adds
+// in the same order into its shift; the shift of round r and its sums are in
+// slot r & 1, so that no block of a round writes what another reads.
 constexpr int kRefineThreads = 256;
 constexpr int kRefineMaxBlocks = 304;
+constexpr int kRefineLanes = 8;
+constexpr int kState = 8;  // doubles of a slot: shift (3), integer-shift flag, matched count
 
 __global__ void k_refine_init(const unsigned long long *__restrict__ best, int o1, int o2, int sb0, int sb1,
                               int sb2, int resc, double *__restrict__ state) {
@@ -215,98 +296,147 @@ __global__ void k_refine_init(const unsigned long long *__restrict__ best, int o
     state[4] = 0.0;
 }
 
+// the state after a round: its predecessor `prev` and the blocks' sums, added by
+// one warp in a fixed order (s is shared memory of kState doubles; ends with a
+// barrier)
+__device__ __forceinline__ void refine_state(const double *__restrict__ prev, const double *__restrict__ parts, int nblocks,
+                                             double *s) {
+    if (threadIdx.x < 32) {
+        const int k = threadIdx.x & 3;
+        double t = 0;
+        for (int b0 = threadIdx.x >> 2; b0 < nblocks; b0 += 64) {
+            double v[8];  // loads first: the additions wait for them once
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = b0 + 8 * u < nblocks ? parts[(b0 + 8 * u) * 4 + k] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) t += v[u];
+        }
+        for (int o = 4; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        const double cnt = __shfl_sync(0xffffffffu, t, 3);
+        // no point kept: the shift stays (align.py:72-74)
+        if (threadIdx.x < 3) s[k] = cnt > 0 ? (double)(float)(t / cnt) : prev[k];
+        if (threadIdx.x == 3) {
+            s[3] = cnt > 0 ? 0.0 : prev[3];
+            s[4] = cnt;
+        }
+    }
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(kRefineThreads)
 k_refine_round(const float *__restrict__ X, const int *__restrict__ n_p, const float *__restrict__ gp,
                const int *__restrict__ gidx, const int *__restrict__ gstart, int gd0, int gd1, int gd2, float lo0,
-               float lo1, float lo2, float cs, int reach, double dist_th, const double *__restrict__ state,
-               double *__restrict__ parts) {
+               float lo1, float lo2, float cs, double dist_th, int round, double *__restrict__ states,
+               double *__restrict__ parts_all) {
+    __shared__ double st[kState], wsum[kRefineThreads / 32][4];
+    double *parts = parts_all + (round & 1) * 4 * kRefineMaxBlocks;
+    if (round == 0) {
+        if (threadIdx.x < 4) st[threadIdx.x] = states[threadIdx.x];
+        __syncthreads();
+    } else {
+        refine_state(states + ((round - 1) & 1) * kState, parts_all + ((round - 1) & 1) * 4 * kRefineMaxBlocks, gridDim.x,
+                     st);
+        if (blockIdx.x == 0 && threadIdx.x < 5) states[(round & 1) * kState + threadIdx.x] = st[threadIdx.x];
+    }
     const int n = *n_p;
-    const bool tint = state[3] != 0.0;
-    const double tz0 = state[0], tz1 = state[1], tz2 = state[2];
+    const bool tint = st[3] != 0.0;
+    const double tz0 = st[0], tz1 = st[1], tz2 = st[2];
     const float t0 = (float)tz0, t1 = (float)tz1, t2 = (float)tz2;
-    double sz = 0, sx = 0, sy = 0, cnt = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        // XT = X - tzxy: float64 against the integer coarse shift, float32 after
-        double q0, q1, q2;
-        if (tint) {
-            q0 = (double)X[i * 3] - tz0;
-            q1 = (double)X[i * 3 + 1] - tz1;
-            q2 = (double)X[i * 3 + 2] - tz2;
-        } else {
-            q0 = (double)(X[i * 3] - t0);
-            q1 = (double)(X[i * 3 + 1] - t1);
-            q2 = (double)(X[i * 3 + 2] - t2);
-        }
-        const int c0 = (int)floor((q0 - lo0) / cs), c1 = (int)floor((q1 - lo1) / cs), c2 = (int)floor((q2 - lo2) / cs);
+    const float radius = (float)dist_th, inv = 1.f / cs;
+    double sum[4] = {0, 0, 0, 0};
+    const int sub = threadIdx.x % kRefineLanes;
+    const int pb = kRefineThreads / kRefineLanes;  // points of a block at a time
+    for (int i0 = blockIdx.x * pb; i0 < n; i0 += gridDim.x * pb) {
+        const int i = i0 + threadIdx.x / kRefineLanes;
         double bd = 1e300;
         int bj = 0x7fffffff, bk = -1;
-        for (int a = max(c0 - reach, 0); a <= min(c0 + reach, gd0 - 1); ++a)
-            for (int b = max(c1 - reach, 0); b <= min(c1 + reach, gd1 - 1); ++b) {
-                const int lc = max(c2 - reach, 0), hc = min(c2 + reach, gd2 - 1);
-                if (lc > hc) continue;
-                const long long row = ((long long)a * gd1 + b) * gd2;
-                const int e0 = gstart[row + lc], e1 = gstart[row + hc + 1];
-                for (int k = e0; k < e1; ++k) {
-                    const double d0 = q0 - gp[k * 3], d1 = q1 - gp[k * 3 + 1], d2 = q2 - gp[k * 3 + 2];
-                    const double d = d0 * d0 + d1 * d1 + d2 * d2;
-                    const int j = gidx[k];
-                    if (d < bd || (d == bd && j < bj)) {
-                        bd = d;
-                        bj = j;
-                        bk = k;
+        if (i < n) {
+            const float x0 = X[i * 3], x1 = X[i * 3 + 1], x2 = X[i * 3 + 2];
+            // the cells within the radius along an axis: the reach is widened
+            // by 1e-5 of the coordinates and 0.01, over 40 float roundings each
+            int c[3][2];
+            auto cells = [&](float x, float t, float lo, int gd, int (&r)[2]) {
+                const float w = radius + 0.01f + 1e-5f * (fabsf(x) + fabsf(t) + fabsf(lo)), q = x - t - lo;
+                r[0] = max(0, (int)floorf(fminf(fmaxf((q - w) * inv - 0.01f, -1.f), 2e9f)));
+                r[1] = min(gd - 1, (int)floorf(fminf(fmaxf((q + w) * inv + 0.01f, -1.f), 2e9f)));
+            };
+            cells(x0, t0, lo0, gd0, c[0]);
+            cells(x1, t1, lo1, gd1, c[1]);
+            cells(x2, t2, lo2, gd2, c[2]);
+            const int nb = c[1][1] - c[1][0] + 1;
+            if (c[0][0] <= c[0][1] && nb > 0 && c[2][0] <= c[2][1])
+                for (int r = sub; r < (c[0][1] - c[0][0] + 1) * nb; r += kRefineLanes) {
+                    const long long row = ((long long)(c[0][0] + r / nb) * gd1 + c[1][0] + r % nb) * gd2;
+                    const int e0 = gstart[row + c[2][0]], e1 = gstart[row + c[2][1] + 1];
+                    for (int k = e0; k < e1; ++k) {
+                        // XT = X - tzxy: float64 against the integer coarse
+                        // shift, float32 after
+                        const double q0 = tint ? (double)x0 - tz0 : (double)(x0 - t0);
+                        const double q1 = tint ? (double)x1 - tz1 : (double)(x1 - t1);
+                        const double q2 = tint ? (double)x2 - tz2 : (double)(x2 - t2);
+                        const double d0 = q0 - gp[k * 3], d1 = q1 - gp[k * 3 + 1], d2 = q2 - gp[k * 3 + 2];
+                        const double d = d0 * d0 + d1 * d1 + d2 * d2;
+                        const int j = gidx[k];
+                        if (d < bd || (d == bd && j < bj)) {
+                            bd = d;
+                            bj = j;
+                            bk = k;
+                        }
                     }
                 }
+        }
+        for (int o = kRefineLanes / 2; o > 0; o >>= 1) {
+            const double d = __shfl_xor_sync(0xffffffffu, bd, o);
+            const int j = __shfl_xor_sync(0xffffffffu, bj, o), k = __shfl_xor_sync(0xffffffffu, bk, o);
+            if (d < bd || (d == bd && j < bj)) {
+                bd = d;
+                bj = j;
+                bk = k;
             }
-        if (bk >= 0 && sqrt(bd) < dist_th) {
+        }
+        if (sub == 0 && bk >= 0 && sqrt(bd) < dist_th) {
             // X_ - X_ref_ in float32, summed in double
-            sz += (double)(X[i * 3] - gp[bk * 3]);
-            sx += (double)(X[i * 3 + 1] - gp[bk * 3 + 1]);
-            sy += (double)(X[i * 3 + 2] - gp[bk * 3 + 2]);
-            cnt += 1;
+            sum[0] += (double)(X[i * 3] - gp[bk * 3]);
+            sum[1] += (double)(X[i * 3 + 1] - gp[bk * 3 + 1]);
+            sum[2] += (double)(X[i * 3 + 2] - gp[bk * 3 + 2]);
+            sum[3] += 1;
         }
     }
-    sz = mm_block_sum(sz);
+    // lanes 0, 8, 16 and 24 hold a warp's sums
+    for (int k = 0; k < 4; ++k) {
+        for (int o = kRefineLanes; o < 32; o <<= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], o);
+        if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5][k] = sum[k];
+    }
     __syncthreads();
-    sx = mm_block_sum(sx);
-    __syncthreads();
-    sy = mm_block_sum(sy);
-    __syncthreads();
-    cnt = mm_block_sum(cnt);
-    if (threadIdx.x == 0) {
-        parts[blockIdx.x * 4 + 0] = sz;
-        parts[blockIdx.x * 4 + 1] = sx;
-        parts[blockIdx.x * 4 + 2] = sy;
-        parts[blockIdx.x * 4 + 3] = cnt;
+    if (threadIdx.x < 4) {
+        double t = 0;
+        for (int w = 0; w < kRefineThreads / 32; ++w) t += wsum[w][threadIdx.x];
+        parts[blockIdx.x * 4 + threadIdx.x] = t;
     }
 }
 
-__global__ void k_refine_update(const double *__restrict__ parts, int nblocks, double *__restrict__ state,
-                                int last, float *__restrict__ out, int *__restrict__ npts) {
-    if (threadIdx.x != 0) return;
-    double s[4] = {0, 0, 0, 0};
-    for (int b = 0; b < nblocks; ++b)
-        for (int k = 0; k < 4; ++k) s[k] += parts[b * 4 + k];
-    state[4] = s[3];
-    if (s[3] > 0) {  // else: no point kept, the shift stays (align.py:72-74)
-        for (int k = 0; k < 3; ++k) state[k] = (double)(float)(s[k] / s[3]);
-        state[3] = 0.0;
-    }
-    if (last) {
-        for (int k = 0; k < 3; ++k) out[k] = (float)state[k];
-        npts[0] = (int)state[4];
-        npts[1] = (int)state[3];
+// the shift after the last round (index `round`), the matched count and the flag
+__global__ void k_refine_last(const double *__restrict__ states, const double *__restrict__ parts_all, int nblocks, int round,
+                              float *__restrict__ out, int *__restrict__ npts) {
+    __shared__ double st[kState];
+    refine_state(states + (round & 1) * kState, parts_all + (round & 1) * 4 * kRefineMaxBlocks, nblocks, st);
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 3; ++k) out[k] = (float)st[k];
+        npts[0] = (int)st[4];
+        npts[1] = (int)st[3];
     }
 }
 
 struct Splat {
     int shape[3];
-    int nvox;
+    bool any;  // voxels survive the trim
 };
 
-// threshold + splat of a point set; fills vox (device, capacity n) and returns shape/nvox on the host
-int splat(const float *pts_dev, const int *n_dev, int n_host, int resc, int trim, int *iv, int *keep, int *mm,
-          int *kmax, unsigned char **grid_buf, size_t *grid_bytes, int *vox, int *nvox_dev, int *h_small,
-          Splat *out, cudaStream_t st) {
+// splat of a point set: its unique voxels as rows in w.rows, w.xs and w.ys, their extents on the host
+int splat(MmDriftWork &w, const int *n_dev, int n_host, int resc, int trim, int *mm, int *kmax, Splat *out,
+          cudaStream_t st) {
+    const float *pts_dev = w.pts;
+    int *iv = w.iv, *keep = w.keep, *h_small = w.h_small;
     const int init[9] = {INT_MAX, INT_MAX, INT_MAX, INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN, INT_MIN};
     MM_CUDA_TRY(cudaMemcpyAsync(mm, init, sizeof(int) * 6, cudaMemcpyHostToDevice, st));
     MM_CUDA_TRY(cudaMemcpyAsync(kmax, init + 6, sizeof(int) * 3, cudaMemcpyHostToDevice, st));
@@ -319,30 +449,40 @@ int splat(const float *pts_dev, const int *n_dev, int n_host, int resc, int trim
     MM_CUDA_TRY(cudaStreamSynchronize(st));
     if (h_small[0] == INT_MIN) {  // nothing survives the trim: a (1,1,1) zero image (align.py:51-53)
         out->shape[0] = out->shape[1] = out->shape[2] = 1;
-        out->nvox = 0;
+        out->any = false;
         return MM_OK;
     }
     for (int c = 0; c < 3; ++c) out->shape[c] = h_small[c] + 1;
     MM_REQUIRE(out->shape[0] > 0 && out->shape[1] > 0 && out->shape[2] > 0, "negative splat extent");
     const size_t total = (size_t)out->shape[0] * out->shape[1] * out->shape[2];
-    if (*grid_bytes < total) {
-        if (*grid_buf) cudaFree(*grid_buf);
-        *grid_buf = nullptr;
-        *grid_bytes = 0;
-        MM_CUDA_TRY(cudaMalloc(grid_buf, total));
-        *grid_bytes = total;
+    if (w.grid_bytes < total) {
+        if (w.grid) cudaFree(w.grid);
+        w.grid = nullptr;
+        w.grid_bytes = 0;
+        MM_CUDA_TRY(cudaMalloc(&w.grid, total));
+        w.grid_bytes = total;
     }
-    MM_CUDA_TRY(cudaMemsetAsync(*grid_buf, 0, total, st));
+    MM_REQUIRE((long long)out->shape[0] * out->shape[1] < (1LL << 31) - 64, "splat image of too many rows");
+    const int nrows = out->shape[0] * out->shape[1];
+    if (w.rows_cap < (size_t)nrows + 1) {
+        cudaFree(w.rows);
+        w.rows = nullptr;
+        w.rows_cap = 0;
+        MM_CUDA_TRY(cudaMalloc(&w.rows, sizeof(int) * ((size_t)nrows + 1)));
+        w.rows_cap = (size_t)nrows + 1;
+    }
+    MM_CUDA_TRY(cudaMemsetAsync(w.grid, 0, total, st));
     MM_CUDA_TRY(cudaMemcpyAsync(mm, out->shape, sizeof(int) * 3, cudaMemcpyHostToDevice, st));
-    k_mark<<<g, 256, 0, st>>>(iv, keep, n_dev, mm, *grid_buf);
+    k_mark<<<g, 256, 0, st>>>(iv, keep, n_dev, mm, w.grid);
     MM_CHECK_LAUNCH();
-    MM_CUDA_TRY(cudaMemsetAsync(nvox_dev, 0, sizeof(int), st));
-    const int gg = (int)((total + 255) / 256 < 152 * 16 ? (total + 255) / 256 : 152 * 16);
-    k_grid_list<<<gg, 256, 0, st>>>(*grid_buf, (long long)total, out->shape[1], out->shape[2], vox, nvox_dev);
+    const int gr = nrows / 8 + 1 < 152 * 8 ? nrows / 8 + 1 : 152 * 8;
+    k_row_count<<<gr, 256, 0, st>>>(w.grid, nrows, out->shape[2], w.rows);
     MM_CHECK_LAUNCH();
-    MM_CUDA_TRY(cudaMemcpyAsync(h_small, nvox_dev, sizeof(int), cudaMemcpyDeviceToHost, st));
-    MM_CUDA_TRY(cudaStreamSynchronize(st));
-    out->nvox = h_small[0];
+    k_row_scan<<<1, 1024, 0, st>>>(w.rows, nrows);
+    MM_CHECK_LAUNCH();
+    k_row_fill<<<gr, 256, 0, st>>>(w.grid, nrows, out->shape[1], out->shape[2], w.rows, w.xs, w.ys);
+    MM_CHECK_LAUNCH();
+    out->any = true;
     return MM_OK;
 }
 
@@ -354,26 +494,28 @@ int work_reserve(MmDriftWork &w, size_t n) {
     cudaFree(w.pts);
     cudaFree(w.iv);
     cudaFree(w.keep);
-    cudaFree(w.vox);
-    w.pts = nullptr; w.iv = w.keep = w.vox = nullptr;
+    cudaFree(w.xs);
+    cudaFree(w.ys);
+    w.pts = nullptr; w.iv = w.keep = w.xs = w.ys = nullptr;
     w.cap = 0;
     MM_CUDA_TRY(cudaMalloc(&w.pts, n * 3 * sizeof(float)));
     MM_CUDA_TRY(cudaMalloc(&w.iv, n * 3 * sizeof(int)));
     MM_CUDA_TRY(cudaMalloc(&w.keep, n * sizeof(int)));
-    MM_CUDA_TRY(cudaMalloc(&w.vox, n * 3 * sizeof(int)));
+    MM_CUDA_TRY(cudaMalloc(&w.xs, n * sizeof(int)));
+    MM_CUDA_TRY(cudaMalloc(&w.ys, n * sizeof(int)));
     w.cap = n;
     return MM_OK;
 }
 
 void work_free(MmDriftWork &w) {
-    cudaFree(w.pts); cudaFree(w.iv); cudaFree(w.keep); cudaFree(w.vox); cudaFree(w.small);
-    cudaFree(w.grid); cudaFree(w.hist);
+    cudaFree(w.pts); cudaFree(w.iv); cudaFree(w.keep); cudaFree(w.xs); cudaFree(w.ys); cudaFree(w.small);
+    cudaFree(w.grid); cudaFree(w.rows);
     if (w.h_small) cudaFreeHost(w.h_small);
     w = MmDriftWork();
 }
 
 // small-buffer slots (ints) inside Work::small
-enum { SM_N = 0, SM_MM = 1, SM_KMAX = 8, SM_NVOX = 12, SM_NPTS = 14, SM_BEST = 16, SM_OUT = 20 };
+enum { SM_N = 0, SM_MM = 1, SM_KMAX = 8, SM_NPTS = 14, SM_BEST = 16, SM_OUT = 20 };
 
 // The cell grid of the reference points (host-side counting sort, points in
 // index order within a cell), and the refinement's small device state.
@@ -421,8 +563,8 @@ int cell_grid_build(MmCellGrid &g, const float *pts_dev, int n, float cs_min, cu
     MM_CUDA_TRY(cudaMalloc(&g.start, sizeof(int) * (ncell + 1)));
     MM_CUDA_TRY(cudaMalloc(&g.pts, sizeof(float) * 3 * n));
     MM_CUDA_TRY(cudaMalloc(&g.idx, sizeof(int) * n));
-    MM_CUDA_TRY(cudaMalloc(&g.state, sizeof(double) * 8));
-    MM_CUDA_TRY(cudaMalloc(&g.parts, sizeof(double) * 4 * kRefineMaxBlocks));
+    MM_CUDA_TRY(cudaMalloc(&g.state, sizeof(double) * 2 * kState));
+    MM_CUDA_TRY(cudaMalloc(&g.parts, sizeof(double) * 2 * 4 * kRefineMaxBlocks));
     MM_CUDA_TRY(cudaMemcpyAsync(g.start, start.data(), sizeof(int) * (ncell + 1), cudaMemcpyHostToDevice, st));
     MM_CUDA_TRY(cudaMemcpyAsync(g.pts, sp.data(), sizeof(float) * 3 * n, cudaMemcpyHostToDevice, st));
     MM_CUDA_TRY(cudaMemcpyAsync(g.idx, idx.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
@@ -445,7 +587,7 @@ extern "C" int mm_aligner_create(const float *X_ref, int n, int cols, int64_t ld
     cudaStream_t st = (cudaStream_t)stream;
     mm_aligner *S = new mm_aligner();
     S->pts = nullptr;
-    S->vox = nullptr;
+    S->rows = S->ys = nullptr;
     S->resc = resc;
     S->trim = trim;
     S->th = th;
@@ -472,26 +614,36 @@ extern "C" int mm_aligner_create(const float *X_ref, int n, int cols, int64_t ld
     }
     S->n = nkeep;
     Splat sp;
-    rc = splat(w.pts, w.small + SM_N, nkeep, resc, trim, w.iv, w.keep, w.small + SM_MM, w.small + SM_KMAX, &w.grid,
-               &w.grid_bytes, w.vox, w.small + SM_NVOX, w.h_small, &sp, st);
+    rc = splat(w, w.small + SM_N, nkeep, resc, trim, w.small + SM_MM, w.small + SM_KMAX, &sp, st);
     if (rc) { work_free(w); delete S; return rc; }
     for (int c = 0; c < 3; ++c) S->shape[c] = sp.shape[c];
-    S->nvox = sp.nvox;
-    // keep the reference points and voxels in buffers of their own
+    const size_t nrows = (size_t)sp.shape[0] * sp.shape[1];
+    w.h_small[0] = 0;
+    if (sp.any && (cudaMemcpyAsync(w.h_small, w.rows + nrows, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                   cudaStreamSynchronize(st) != cudaSuccess)) {
+        work_free(w); delete S;
+        mm_set_error("aligner: splat failed");
+        return MM_EDEVICE;
+    }
+    S->nvox = w.h_small[0];
+    // keep the reference points and voxel rows in buffers of their own
     S->pts = nullptr;
-    S->vox = nullptr;
     if (cudaMalloc(&S->pts, sizeof(float) * 3 * nkeep) != cudaSuccess ||
-        cudaMalloc(&S->vox, sizeof(int) * 3 * (sp.nvox > 0 ? sp.nvox : 1)) != cudaSuccess) {
+        cudaMalloc(&S->rows, sizeof(int) * (nrows + 1)) != cudaSuccess ||
+        cudaMalloc(&S->ys, sizeof(int) * (S->nvox > 0 ? S->nvox : 1)) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(S->pts); cudaFree(S->vox); work_free(w); delete S;
+        cudaFree(S->pts); cudaFree(S->rows); cudaFree(S->ys); work_free(w); delete S;
         mm_set_error("aligner: out of device memory");
         return MM_ENOMEM;
     }
     cudaMemcpyAsync(S->pts, w.pts, sizeof(float) * 3 * nkeep, cudaMemcpyDeviceToDevice, st);
-    if (sp.nvox) cudaMemcpyAsync(S->vox, w.vox, sizeof(int) * 3 * sp.nvox, cudaMemcpyDeviceToDevice, st);
+    if (S->nvox) {
+        cudaMemcpyAsync(S->rows, w.rows, sizeof(int) * (nrows + 1), cudaMemcpyDeviceToDevice, st);
+        cudaMemcpyAsync(S->ys, w.ys, sizeof(int) * S->nvox, cudaMemcpyDeviceToDevice, st);
+    }
     MM_CUDA_TRY(cudaStreamSynchronize(st));
     if ((rc = cell_grid_build(S->cg, S->pts, nkeep, (float)resc, st))) {
-        cell_grid_free(S->cg); cudaFree(S->pts); cudaFree(S->vox); work_free(w); delete S;
+        cell_grid_free(S->cg); cudaFree(S->pts); cudaFree(S->rows); cudaFree(S->ys); work_free(w); delete S;
         return rc;
     }
     *out = S;
@@ -502,7 +654,8 @@ extern "C" int mm_aligner_destroy(mm_aligner *S) {
     if (!S) return MM_OK;
     cudaDeviceSynchronize();
     cudaFree(S->pts);
-    cudaFree(S->vox);
+    cudaFree(S->rows);
+    cudaFree(S->ys);
     work_free(S->w);
     cell_grid_free(S->cg);
     delete S;
@@ -525,7 +678,7 @@ extern "C" int mm_aligner_translation(mm_aligner *S, const float *X, int n, int 
     const mm_aligner &A = *S;
     MmDriftWork &w = S->w;
     cudaStream_t st = (cudaStream_t)stream;
-    int rc = work_reserve(w, (size_t)(n > A.nvox ? n : A.nvox));
+    int rc = work_reserve(w, (size_t)n);
     if (rc) return rc;
     // get_best_translation_points: threshold on the last column (align.py:97-101)
     int nm = 0;
@@ -538,55 +691,36 @@ extern "C" int mm_aligner_translation(mm_aligner *S, const float *X, int n, int 
     } else {
         MM_CUDA_TRY(cudaMemsetAsync(w.small + SM_N, 0, sizeof(int), st));
     }
-    Splat sp = {{1, 1, 1}, 0};
+    Splat sp = {{1, 1, 1}, false};
     if (nm > 0) {
-        rc = splat(w.pts, w.small + SM_N, nm, A.resc, A.trim, w.iv, w.keep, w.small + SM_MM, w.small + SM_KMAX,
-                   &w.grid, &w.grid_bytes, w.vox, w.small + SM_NVOX, w.h_small, &sp, st);
+        rc = splat(w, w.small + SM_N, nm, A.resc, A.trim, w.small + SM_MM, w.small + SM_KMAX, &sp, st);
         if (rc) return rc;
     }
     // full correlation shape sa + sb - 1
     const int o0 = sp.shape[0] + A.shape[0] - 1, o1 = sp.shape[1] + A.shape[1] - 1, o2 = sp.shape[2] + A.shape[2] - 1;
-    const size_t total = (size_t)o0 * o1 * o2;
-    if (w.hist_bytes < total * sizeof(int)) {
-        cudaFree(w.hist);
-        w.hist = nullptr;
-        w.hist_bytes = 0;
-        MM_CUDA_TRY(cudaMalloc(&w.hist, total * sizeof(int)));
-        w.hist_bytes = total * sizeof(int);
-    }
-    MM_CUDA_TRY(cudaMemsetAsync(w.hist, 0, total * sizeof(int), st));
-    MM_CUDA_TRY(cudaMemcpyAsync(w.small + SM_NVOX, &sp.nvox, sizeof(int), cudaMemcpyHostToDevice, st));
-    const long long pairs = (long long)sp.nvox * A.nvox;
-    if (pairs > 0) {
-        const int g = (int)((pairs + 255) / 256 < 152 * 32 ? (pairs + 255) / 256 : 152 * 32);
-        k_pair_hist<<<g, 256, 0, st>>>(w.vox, w.small + SM_NVOX, A.vox, A.nvox, A.shape[0] - 1, A.shape[1] - 1,
-                                       A.shape[2] - 1, o1, o2, w.hist);
-        MM_CHECK_LAUNCH();
-    }
     unsigned long long *best = reinterpret_cast<unsigned long long *>(w.small + SM_BEST);
     MM_CUDA_TRY(cudaMemsetAsync(best, 0, sizeof(unsigned long long), st));
-    const int ga = (int)((total + 255) / 256 < 152 * 16 ? (total + 255) / 256 : 152 * 16);
-    k_argmax<<<ga, 256, 0, st>>>(w.hist, (long long)total, best);
+    const CorrShape cs = {{sp.shape[0], sp.shape[1]}, {A.shape[0], A.shape[1]}, o1, o2, A.shape[2] - 1, (long long)o0 * o1};
+    const bool pairs = sp.any && A.nvox > 0;  // none: every count is 0, the first shift is the peak
+    k_corr_rows<<<(unsigned)std::min(cs.nout, 152LL * 32), kCorrThreads, 0, st>>>(pairs ? w.rows : nullptr, w.xs, w.ys,
+                                                                                  A.rows, A.ys, cs, best);
     MM_CHECK_LAUNCH();
     float *outp = reinterpret_cast<float *>(w.small + SM_OUT);
     const MmCellGrid &G = A.cg;
     k_refine_init<<<1, 1, 0, st>>>(best, o1, o2, A.shape[0], A.shape[1], A.shape[2], A.resc, G.state);
     MM_CHECK_LAUNCH();
-    // radius in cells: the largest match radius over the rounds
-    const double rmax = std::max((double)A.resc, (double)target);
-    const int reach = (int)std::ceil(rmax / G.cs);
-    int nb = (nm + kRefineThreads - 1) / kRefineThreads;
+    int nb = mm_cdiv((long)nm * kRefineLanes, kRefineThreads);
     nb = std::max(1, std::min(nb, kRefineMaxBlocks));
     for (int it = 0; it < 5; ++it) {
         // np.linspace(resc, target, 5)
         const double dist_th = (double)A.resc + (double)it * (((double)target - (double)A.resc) / 4.0);
         k_refine_round<<<nb, kRefineThreads, 0, st>>>(w.pts, w.small + SM_N, G.pts, G.idx, G.start, G.dims[0],
-                                                      G.dims[1], G.dims[2], G.lo[0], G.lo[1], G.lo[2], G.cs, reach,
-                                                      dist_th, G.state, G.parts);
-        MM_CHECK_LAUNCH();
-        k_refine_update<<<1, 32, 0, st>>>(G.parts, nb, G.state, it == 4, outp, w.small + SM_NPTS);
+                                                      G.dims[1], G.dims[2], G.lo[0], G.lo[1], G.lo[2], G.cs, dist_th,
+                                                      it, G.state, G.parts);
         MM_CHECK_LAUNCH();
     }
+    k_refine_last<<<1, 32, 0, st>>>(G.state, G.parts, nb, 4, outp, w.small + SM_NPTS);
+    MM_CHECK_LAUNCH();
     MM_CUDA_TRY(cudaMemcpyAsync(w.h_small, outp, sizeof(float) * 3, cudaMemcpyDeviceToHost, st));
     MM_CUDA_TRY(cudaMemcpyAsync(w.h_small + 4, w.small + SM_NPTS, sizeof(int) * 2, cudaMemcpyDeviceToHost, st));
     MM_CUDA_TRY(cudaStreamSynchronize(st));
