@@ -281,9 +281,9 @@ k_maxima(Vols V, float th, int delta, Xform t, uint2 *__restrict__ cand, unsigne
     const bool skip_small = t.div > 0.f && th > 0.f;
     // the two-sign pass with th >= 0 (not NaN): one queue round per voxel
     const bool excl = both && th >= 0.f;
-    const bool skip_chunk = skip_small || (t.div == 0.f && th >= 0.f);
+    const bool skip_pieces = skip_small || (t.div == 0.f && th >= 0.f);
     const float lo = skip_small ? th * t.div * (1.f - 0x1p-18f) : 0.f;
-    const float chunk_th = skip_small ? lo : th;
+    const float piece_th = skip_small ? lo : th;
     const unsigned keep_bits = skip_small || both ? 0x7fffffffu : 0xffffffffu;  // |value|, or value
     const unsigned flip_bits = !(skip_small || both) && t.neg ? 0x80000000u : 0u;
     unsigned *my_k = qk[warp];
@@ -302,18 +302,20 @@ k_maxima(Vols V, float th, int delta, Xform t, uint2 *__restrict__ cand, unsigne
                 const int y = y0 + 32 * k + (int)lane;
                 vals[k] = y < yhi ? rp[y] : 0.f;
             }
-            // a chunk without a value the threshold lets pass (most chunks of a
-            // volume thresholded above its noise) ends here.  With a divisor the
-            // test is the one that spares the quotient; without one the value
-            // itself is compared, in the sign asked for (a NaN passes).  DAPI
-            // block of 50 x 1500 x 1302: 0.74 -> 0.61 ms with its fits,
-            // a colour of 25 tiles 0.36 -> 0.24
-            if (skip_chunk) {
-                bool some = false;
+            // the 32-voxel pieces with a value the threshold lets pass: the others
+            // (most, in a volume thresholded above its noise) end here.  With a
+            // divisor the test is the one that spares the quotient; without one
+            // the value itself is compared, in the sign asked for (a NaN passes).
+            // DAPI block of 50 x 1500 x 1302: 0.74 -> 0.59 ms with its fits, a
+            // colour of 25 tiles 0.36 -> 0.23
+            unsigned pieces = 0xffffffffu;
+            if (skip_pieces) {
+                pieces = 0;
 #pragma unroll
                 for (int k = 0; k < kMaxY; ++k)
-                    some |= !(__uint_as_float((__float_as_uint(vals[k]) & keep_bits) ^ flip_bits) <= chunk_th);
-                if (!__any_sync(0xffffffffu, some)) continue;
+                    if (!(__uint_as_float((__float_as_uint(vals[k]) & keep_bits) ^ flip_bits) <= piece_th)) pieces |= 1u << k;
+                pieces = __reduce_or_sync(0xffffffffu, pieces);
+                if (!pieces) continue;
             }
             // queue the voxels above the threshold (maxima.cu:19; a NaN
             // threshold admits every voxel) whose y neighbours held by the
@@ -321,6 +323,7 @@ k_maxima(Vols V, float th, int delta, Xform t, uint2 *__restrict__ cand, unsigne
             // fails the test anyway, so only the others need it
 #pragma unroll
             for (int k = 0; k < kMaxY; ++k) {
+                if (!(pieces >> k & 1)) continue;
                 const int y = y0 + 32 * k + (int)lane;
                 // a value below the threshold enters only as a y neighbour,
                 // which it cannot be above, so 0 stands for it there
@@ -424,6 +427,7 @@ k_fit(Vols V, const uint2 *__restrict__ cand, const unsigned *__restrict__ ncand
       unsigned *__restrict__ out_count, int keep_filter) {
     __shared__ float gtab[kSphereCap];
     __shared__ char4 otab[kSphereCap];
+    __shared__ double inv_full;  // 1 / samples of a spot that has them all
     t = xf_resolve(t);
     const unsigned lane = threadIdx.x & 31;
     const unsigned nc = min(*ncand, cap);
@@ -432,6 +436,7 @@ k_fit(Vols V, const uint2 *__restrict__ cand, const unsigned *__restrict__ ncand
     const int nsamp = table ? g_fit_sphere_n[delta_fit] : side * side * side;
     const int df2 = delta_fit * delta_fit;
     const float gz = 2 * sigmaZ * sigmaZ, gxy = 2 * sigmaXY * sigmaXY;
+    if (threadIdx.x == 0) inv_full = 1.0 / (double)nsamp;
     if (table)
         for (int i = threadIdx.x; i < nsamp; i += blockDim.x) {
             const char4 o = g_fit_sphere[delta_fit][i];
@@ -532,17 +537,28 @@ k_fit(Vols V, const uint2 *__restrict__ cand, const unsigned *__restrict__ ncand
         }
         warp_sum16(acc, lane);
         for (int o = 16; o > 0; o >>= 1) vmin = fminf(vmin, __shfl_xor_sync(0xffffffffu, vmin, o));
-        if (lane != 0 || acc[0] == 0.f) continue;
+        if (acc[0] == 0.f) continue;  // all lanes hold the sums
         // Only the variances and covariances cancel (mean square minus squared
         // mean of the shifted values): they are formed in double precision; the
         // quotients, roots and the centroid in float, as the reference does.
-        const double N = acc[0], invN = 1.0 / N;
-        const double mg = acc[3] * invN, mv = acc[1] * invN, mr = acc[6] * invN;
-        const float varg = (float)fmax(acc[4] * invN - mg * mg, 0.0);
-        const float varv = (float)fmax(acc[2] * invN - mv * mv, 0.0);
-        const float varr = (float)fmax(acc[7] * invN - mr * mr, 0.0);
-        const float covg_v = (float)(acc[5] * invN - mv * mg);
-        const float covg_r = (float)(acc[8] * invN - mr * mg);
+        // Lanes 0 .. 4 form one each, since a warp's double instruction takes
+        // sixteen cycles of the SM whichever lanes are active (26 K spots of 123
+        // samples: 71 -> 51 us).
+        const double invN = acc[0] == (float)nsamp ? inv_full : 1.0 / (double)acc[0];
+        const bool cv2 = lane == 3 || lane == 4;
+        const float mq = lane == 0 || cv2 ? acc[3] : lane == 1 ? acc[1] : acc[6];
+        const float mp = lane == 0 ? acc[3] : (lane == 1 || lane == 3) ? acc[1] : acc[6];
+        const float mm = lane == 0 ? acc[4] : lane == 1 ? acc[2] : lane == 2 ? acc[7] : lane == 3 ? acc[5] : acc[8];
+        double dd = 0.0;
+        if (lane < 5) {
+            dd = (double)mm * invN - ((double)mp * invN) * ((double)mq * invN);
+            if (!cv2) dd = fmax(dd, 0.0);
+        }
+        const float cc = (float)dd;
+        const float varg = __shfl_sync(0xffffffffu, cc, 0), varv = __shfl_sync(0xffffffffu, cc, 1);
+        const float varr = __shfl_sync(0xffffffffu, cc, 2), covg_v = __shfl_sync(0xffffffffu, cc, 3);
+        const float covg_r = __shfl_sync(0xffffffffu, cc, 4);
+        if (lane != 0) continue;
         const float stdg = sqrtf(varg);
         float stdv = sqrtf(varv), stdr = sqrtf(varr);
         if (!(stdv > 0.f)) stdv = 1.f;
