@@ -47,7 +47,7 @@ namespace {
 constexpr int kTI = 5;      // rows of a thread, and the unroll of the column loop
 // threads of a CTA at most, and CTAs per SM that the registers are shared out for
 constexpr int zth_ctas(int tt, int pb) { return tt == 5 && pb == 8 ? 1 : 2; }
-constexpr int zth_max_threads(int tt, int pb) { return tt == 5 && pb == 8 ? 448 : 256; }
+constexpr int zth_max_threads(int tt, int pb) { return 512 / zth_ctas(tt, pb); }
 constexpr unsigned kWaitPolls = 1u << 24;
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
@@ -184,13 +184,14 @@ k_zth_apply(float2 *__restrict__ S, const __grid_constant__ CUtensorMap wmapA, c
         return;
     }
     const int lane = tid & 31, warp = tid >> 5;
-    const int ncw = (PB * nig * a.ntg + 31) / 32;  // compute warps; warp ncw produces
+    const int ncw = (int)(blockDim.x >> 5) - 1;          // compute warps; warp ncw produces
+    const int units = (PB * nig * a.ntg + 31) / 32;      // warp units of an item
     if (tid == 0) {
         for (int b = 0; b < 2; ++b) {
             // the producer warp's 32 copy arrivals and the arrive that counts
             // the TMA bytes
             mbar_init(&full[b], 33);
-            mbar_init(&empty[b], ncw);
+            mbar_init(&empty[b], units);
         }
         unit_next = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -243,21 +244,21 @@ k_zth_apply(float2 *__restrict__ S, const __grid_constant__ CUtensorMap wmapA, c
         return;
     }
 
-    // An item's threads (PB x nig x ntg) come in ncw warp units: unit u
-    // is threads 32u .. 32u + 31 of the item.  The compute warps take the
-    // units in order from a shared counter, so a warp on a less loaded SM
-    // sub-partition takes more of them (ncw warps of two CTAs do not divide
-    // evenly over four sub-partitions).  The parity wait below passes on this
+    // An item's threads (PB x nig x ntg) come in warp units: unit u is threads
+    // 32u .. 32u + 31 of the item.  The compute warps (between units and 2 units
+    // of them) take the units in order from a shared counter, so a warp on a
+    // less loaded SM sub-partition takes more of them, and warps beyond an
+    // item's units start the next item's.  The parity wait below passes on this
     // item's own phase: to pass on item it - 2's, a warp would have to take a
     // unit of item it while that item's buffer is unfilled.  The producer
     // fills in order, so no unit of items it - 2 and it - 1 could have
-    // finished, and their 2 ncw units would occupy more warps than the CTA's
-    // ncw.
+    // finished, and their 2 units would occupy 2 units warps besides the taker,
+    // more than the CTA has.
     for (;;) {
         unsigned sq = 0;
         if (lane == 0) sq = atomicAdd(&unit_next, 1u);
         sq = __shfl_sync(0xffffffffu, sq, 0);
-        const int it = (int)(sq / (unsigned)ncw), unit = (int)(sq - (unsigned)it * (unsigned)ncw);
+        const int it = (int)(sq / (unsigned)units), unit = (int)(sq - (unsigned)it * (unsigned)units);
         const long long item_ll = blockIdx.x + (long long)it * gridDim.x;
         if (item_ll >= a.nitems) break;
         const int item = (int)item_ll;
@@ -434,10 +435,8 @@ int make_map(CUtensorMap *m, const void *base, int rank, const cuuint64_t *dims,
     return MM_OK;
 }
 
-// the compute warps (threads PB x ceil(Z / kTI) x ntg, rounded up to whole
-// warps) and the producer warp
-int zth_threads(int Z, int pb, int ntg) { return ((pb * ((Z + kTI - 1) / kTI) * ntg + 31) / 32 + 1) * 32; }
-
+// warp units of an item (threads PB x ceil(Z / kTI) x ntg)
+int zth_units(int Z, int pb, int ntg) { return (pb * ((Z + kTI - 1) / kTI) * ntg + 31) / 32; }
 // staged row of w[0]: the rows -(2Z-2) .. -1 rounded up to a multiple of four,
 // so that the second kernel box starts on a 128-byte boundary
 int zth_ka(int Z) { return (2 * Z - 2 + 3) & ~3; }
@@ -468,7 +467,7 @@ struct ZthPlan {
     int tt, pb, nchunks, ntc, ntg;
 };
 bool zth_fits(int Z, int pb, int tt, int ntg) {
-    return zth_threads(Z, pb, ntg) <= zth_max_threads(tt, pb) &&
+    return (zth_units(Z, pb, ntg) + 1) * 32 <= zth_max_threads(tt, pb) &&
            2 * zth_bufstride(Z, pb, ntg * tt, nullptr) + zth_zero_bytes(Z, pb) <= kSmemMax / zth_ctas(tt, pb);
 }
 bool zth_split(int Z, int nt, int tt, int pb, ZthPlan *pl) {
@@ -485,25 +484,53 @@ bool zth_split(int Z, int nt, int tt, int pb, ZthPlan *pl) {
 }
 // Measured at P = 678 (ms per launch; the per-tile form, or for Z = 37 the
 // direct sum, in brackets): Z = 50, 2 tiles, 16 frequencies of 2 tiles a thread
-// 0.32 [0.40]; 3 tiles, 8 x 3 0.50 [0.56]; 4 tiles, 8 x 2 0.59, 8 x 5 0.67
-// [0.75]; 6 tiles, 8 x 3 0.80, 8 x 5 1.06 [1.12]; 9 tiles, 8 x 5 1.12, 8 x 3
-// 1.25, 4 x 5 1.20 [2.27 at zpad 24]; 16 tiles, 4 x 5 2.06, 8 x 5 2.11; 25
-// tiles, 4 x 5 2.69, 8 x 5 2.75; Z = 37, 9 tiles, 8 x 5 0.70 [2.14], 25 tiles,
-// 8 x 5 1.78, 4 x 5 2.06.  So few tiles take as many per thread as leave no
-// place empty and wide groups (a row of 8 frequencies is 64 bytes); from 11
-// tiles on the groups are narrow for a depth of whole row groups, where two CTAs
-// share an SM, and wide for a cut one while a single chunk fits.
+// 0.29 [0.39]; 3 tiles, 8 x 3 0.45 [0.58]; 4 tiles, 8 x 2 0.58, 8 x 5 0.72
+// [0.81]; 6 tiles, 8 x 3 0.75, 8 x 5 1.16 [1.21]; 9 tiles, 8 x 5 1.22, 4 x 5
+// 1.26 [2.46 at zpad 24]; Z = 37, 9 tiles, 8 x 3 0.67, 8 x 5 0.72 [2.3].  So up
+// to ten tiles the groups are wide (a row of 8 frequencies is 64 bytes), and a
+// thread's tiles those with the largest share of products in its work: of its
+// places that hold a tile, of its warps' lanes in use, and of a column's
+// instructions (20 products and 1 load per tile, 15 to form its entries).  More
+// tiles: 5 a thread, on 8 frequencies (25 tiles of Z = 37: 1.78 against 2.05;
+// 20 of Z = 56: 2.81 against 3.06) but for the depth with its own kernel (25
+// tiles of Z = 50: 4 frequencies 2.83, 8 2.94; 16 tiles 1.97 against 2.21).
 bool zth_plan(int Z, int nt, ZthPlan *pl) {
 #ifdef ZTH_FORCE
     return zth_split(Z, nt, g_tt, g_pb, pl);
 #endif
+    if (nt <= 2 && zth_split(Z, nt, nt, 16, pl) && pl->nchunks == 1) return true;
     if (nt <= 10) {
-        const int tt = nt <= 3 ? nt : nt == 4 ? 2 : nt == 6 ? 3 : 5;
-        if (zth_split(Z, nt, tt, nt <= 2 ? 16 : 8, pl) && pl->nchunks == 1) return true;
-    } else if (Z % kTI != 0) {
-        if (zth_split(Z, nt, 5, 8, pl) && pl->nchunks == 1) return true;
+        double best = 0;
+        ZthPlan c;
+        for (int tt : {5, 3, 2}) {
+            if (!zth_split(Z, nt, tt, 8, &c) || c.nchunks != 1) continue;
+            const double lanes = 8.0 * ((Z + kTI - 1) / kTI) * c.ntg / (32.0 * zth_units(Z, 8, c.ntg));
+            const double share = (double)nt / (c.ntg * tt) * lanes * 20.0 * tt / (21.0 * tt + 15.0);
+            if (share > best) {
+                best = share;
+                *pl = c;
+            }
+        }
+        if (best > 0) return true;
+    } else if (Z != 50 && zth_split(Z, nt, 5, 8, pl) && pl->nchunks == 1) {
+        return true;
     }
     return zth_split(Z, nt, 5, 4, pl);
+}
+
+// Threads of a CTA: the producer warp, a compute warp per unit, and more (up to
+// two per unit, see the kernel) as far as the CTAs that fit an SM beside each
+// other leave registers: a warp beyond an item's units starts the next item (6
+// tiles of Z = 50: 0.79 -> 0.75 ms, 16 tiles 2.07 -> 1.97).
+int zth_threads(int Z, const ZthPlan &pl, size_t smem) {
+    const int units = zth_units(Z, pl.pb, pl.ntg);
+    int ctas = 16 / (units + 1);
+    if (ctas > (int)(kSmemMax / smem)) ctas = (int)(kSmemMax / smem);
+    if (ctas < 1) ctas = 1;
+    int w = 16 / ctas - 1;
+    if (w > zth_max_threads(pl.tt, pl.pb) / 32 - 1) w = zth_max_threads(pl.tt, pl.pb) / 32 - 1;
+    if (w > 2 * units) w = 2 * units;
+    return ((w > units ? w : units) + 1) * 32;
 }
 
 const void *zth_kernel(int Z, const ZthPlan &pl) {
@@ -579,7 +606,7 @@ int mm_launch_zth_apply(float2 *S, const float2 *w, int Z, int zpad, int Zp, lon
     a.fresp = fresp;
     a.err = err;
     const size_t sm = 2 * (size_t)a.bufstride + zth_zero_bytes(Z, pl.pb);
-    const int threads = zth_threads(Z, pl.pb, a.ntg);
+    const int threads = zth_threads(Z, pl, sm);
     const void *fn = zth_kernel(Z, pl);
     MM_REQUIRE(fn != nullptr, "z operator: no kernel for %d tiles per thread, %d frequencies", pl.tt, pl.pb);
     if (int rc = mm_set_smem(fn, sm)) return rc;

@@ -605,6 +605,16 @@ def _unit_protocol_run(rng, nwarps, nunits, nitems):
     raise AssertionError("no end")
 
 
+def test_register_z_operator_more_warps_than_units():
+    """The register z operator may run up to twice as many compute warps as an
+    item has units (the warps beyond them start the next item): no wait passes
+    on an earlier phase and nothing deadlocks."""
+    rng = np.random.default_rng(12)
+    for _ in range(300):
+        u = int(rng.integers(1, 9))
+        assert _unit_protocol_run(rng, int(rng.integers(u, 2 * u + 1)), u, int(rng.integers(1, 25))) == []
+
+
 def test_register_z_operator_warp_unit_protocol():
     """The register z operator's compute warps take an item's warp units from
     a shared counter and wait for their buffer with a parity wait only.  With
