@@ -218,6 +218,20 @@ int fill_geom(TileGeom &g, int Z, int X, int Y, long long isz, long long isx, lo
 }
 
 
+// Whether the stitched centres of a field's tiles cover it: each tile's centre
+// reaches to the end of the tile's own span, or of the field.
+bool stitch_covers(const TileGeom &g) {
+    const int nx = (g.X + g.ts - 1) / g.ts;
+    if (g.ntot < nx * g.ny) return false;
+    for (int ix = 0; ix < nx; ++ix)
+        for (int iy = 0; iy < g.ny; ++iy) {
+            const TileDesc d = mm_tile_desc(g, ix * g.ny + iy);
+            const int sx = g.X - d.x < g.ts ? g.X - d.x : g.ts, sy = g.Y - d.y < g.ts ? g.Y - d.y : g.ts;
+            if (d.xend - 2 * g.ov < sx || d.yend - 2 * g.ov < sy) return false;
+        }
+    return true;
+}
+
 // Whether a call may fold the blur subtraction into the z step (the
 // spectrum times 1 - D(kx) D(ky), mm_blur_response_get): the z step runs from
 // the z kernel, and every voxel the caller reads lies at least delta (the
@@ -286,10 +300,11 @@ bool fold_allowed(const mm_ctx *c, const TileGeom &g, int blur_radius, const flo
 // runs as a factor of the z step's output (fold_allowed) instead of the y and
 // x box means of the result
 //
-// win: with the blur folded, the caller reads only a window of each tile (a
-// driver's keep band, win >= 0 its reach, or the stitched centre, win == -1):
-// the inverse y pass then transforms and writes only the rows and columns of
-// that window (k_rows_inv_win).  win < -1: whole tiles.
+// win: with no box means left to take on the result (the blur folded, or none
+// asked for), the caller reads only a window of each tile (a driver's keep band,
+// win >= 0 its reach, or the stitched centre, win == -1): the inverse y pass then
+// transforms and writes only the rows and columns of that window.  win < -1:
+// whole tiles.
 int run_tiles(mm_ctx *c, TileGeom g, const void *image, int dtype, const float *flat, const float2 *W,
               const float2 *zop, int blur_radius, float *res_out, float *raw_out, float *stitch, long long osz,
               long long osx, cudaStream_t st, bool fold = false, int win = -2) {
@@ -360,10 +375,11 @@ int run_tiles(mm_ctx *c, TileGeom g, const void *image, int dtype, const float *
         StageTimer t(c, ST_COLS_INV, 2 * spec_b, st);
         if ((rc = mm_launch_cols(S, g.P, g.H, g.H, plane_c, g.nt * g.Z, true, sm->queue, st))) return rc;
     }
-    // with the blur folded and only the centre read, the stitched buffer is
-    // written straight from the inverse pass
-    const bool direct_stitch = fresp && win == -1 && !res_out && stitch;
-    if (fresp && win >= -1 && !res_out) {
+    // with only the centre read, the stitched buffer is written straight from
+    // the inverse pass
+    const bool windowed = rdelta < 0 && win >= -1 && !res_out && g.nt <= MM_MAX_WIN_TILES;
+    const bool direct_stitch = windowed && win == -1 && stitch;
+    if (windowed) {
         StageTimer t(c, ST_ROWS_INV, spec_b + real_b, st);
         if ((rc = mm_launch_rows_inv_win(S, g, win, (float *)res, direct_stitch ? stitch : nullptr, osz, osx,
                                          sm->queue, st)))
@@ -493,8 +509,13 @@ int mm_deconv_tiles(mm_ctx *c, const void *image, int image_dtype, int Z, int X,
     g.nt = tile_count;
     std::lock_guard<std::mutex> lock(c->mu);
     const bool fold = fold_allowed(c, g, blur_radius, (const float2 *)zop, false, 0);
+    // a call that asks for the stitched centres alone, with no box means to take
+    // on the result, reads nothing else of a tile (6 tiles of 50 x 678 x 678
+    // without a blur: 2.00 -> 1.69 ms)
+    const bool centre = stitch_out && !res_out;
     return run_tiles(c, g, image, image_dtype, flat, (const float2 *)W, (const float2 *)zop, blur_radius, res_out,
-                     raw_out, stitch_out, osz, osx, (cudaStream_t)stream, fold);
+                     raw_out, stitch_out, osz, osx, (cudaStream_t)stream, fold,
+                     centre && (fold || blur_radius < 0) ? -1 : -2);
 }
 
 int mm_find_local_maxima(mm_ctx *c, const float *image, int Z, int X, int Y, int64_t isz, int64_t isx,
@@ -564,7 +585,7 @@ static int hyb_pass(mm_ctx *c, const TileGeom &g, int batch, const uint16_t *ima
         // region, maxima.cu scan_range) and reads max(delta, delta_fit) around it
         const int win = delta_fit + 1 + (delta > delta_fit ? delta : delta_fit);
         if ((rc = run_tiles(c, gb, image, MM_DTYPE_U16, flat, (const float2 *)W, (const float2 *)zop, blur_radius,
-                            nullptr, nullptr, nullptr, 0, 0, st, fold, win)))
+                            nullptr, nullptr, nullptr, 0, 0, st, fold, fold ? win : -2)))
             return rc;
         MaximaArgs a = {};
         a.img = (const float *)c->ws[WS_RES];
@@ -686,14 +707,17 @@ static int dapi_pass(mm_ctx *c, const TileGeom &g, int batch, const uint16_t *im
     const int nt = ntiles_of(g);
     const int Z = g.Z, X = g.X, Y = g.Y;
     const long long N = (long long)Z * X * Y;
-    MM_CUDA_TRY(cudaMemsetAsync(buffer, 0, sizeof(float) * N, st));
+    // voxels that no tile writes are zero: those of a field whose tiles leave
+    // gaps (a cut first tile, fewer spectra than tiles), else there are none
+    if (!stitch_covers(g)) MM_CUDA_TRY(cudaMemsetAsync(buffer, 0, sizeof(float) * N, st));
     for (int t0 = 0; t0 < nt; t0 += batch) {
         TileGeom gb = g;
         gb.t0 = t0;
         gb.nt = (t0 + batch <= nt) ? batch : nt - t0;
         const bool fold = fold_allowed(c, gb, blur_radius, (const float2 *)zop, true, 0);
         if ((rc = run_tiles(c, gb, image, MM_DTYPE_U16, flat, (const float2 *)W, (const float2 *)zop, blur_radius,
-                            nullptr, nullptr, buffer, (long long)X * Y, Y, st, fold, -1)))
+                            nullptr, nullptr, buffer, (long long)X * Y, Y, st, fold,
+                            fold || blur_radius < 0 ? -1 : -2)))
             return rc;
     }
     {

@@ -380,8 +380,7 @@ k_rows_inv(const float2 *__restrict__ S, long long nrows, int H, float *__restri
 // [xlo, xhi) of every plane, in groups of 2 nl rows (a plane's last group is
 // cut at xhi), stores limited to the columns [ylo, yhi).  Rows and columns
 // outside are not written.  The CTAs first tabulate the groups per tile
-// (tiles <= kMaxWinTiles), then walk the groups as k_rows_inv does.
-constexpr int kMaxWinTiles = 256;
+// (tiles <= MM_MAX_WIN_TILES), then walk the groups as k_rows_inv does.
 template <int LMAX>
 __global__ void __launch_bounds__(kRowsInvCfg.threads, kRowsInvCfg.ctas)
 k_rows_inv_win(const float2 *__restrict__ S, TileGeom g, int reach, float *__restrict__ out, FftPlan P, int nl,
@@ -631,7 +630,7 @@ int mm_launch_rows_inv_win(const float2 *S, const TileGeom &g, int reach, float 
     FftPlan P;
     int rc = mm_fft_plan_get(g.P, &P);
     if (rc) return rc;
-    MM_REQUIRE(g.nt <= kMaxWinTiles, "windowed inverse pass takes at most %d tiles per batch", kMaxWinTiles);
+    MM_REQUIRE(g.nt <= MM_MAX_WIN_TILES, "windowed inverse pass takes at most %d tiles per batch", MM_MAX_WIN_TILES);
     if (mm_rows_pfa_takes(P, (long long)g.nt * g.Z * g.P))
         return mm_launch_rows_inv_win_pfa(S, g, reach, out, stitch, osz, osx, P, queue, st);
     const size_t lim = (size_t)fft_smem_limit(kRowsInvCfg);

@@ -199,6 +199,7 @@ int mm_blur_response_get(int P, int delta, const float **out);
 int mm_launch_zfwd(float2 *S, int Zp, int plane, cudaStream_t st);
 int mm_launch_rows_inv(const float2 *S, int nrows, int P, int H, float *out, float *blur, int delta,
                        unsigned *queue, cudaStream_t st);
+#define MM_MAX_WIN_TILES 256  // tiles of a windowed inverse pass
 // the inverse y pass (no blur) over the rows and columns of each tile that the
 // caller reads: reach >= 0, the band [ov - reach, extent - ov + reach) of the
 // hyb keep filter; reach < 0, the stitched centre [ov, extent - ov)

@@ -364,8 +364,6 @@ k_rows_fwd_pfa(TileGeom g, const T *__restrict__ img, const float *__restrict__ 
 // those of the whole-row pass, so the voxels are the same bits, and a tile's
 // lines are numbered through its planes.
 // ---------------------------------------------------------------------------
-constexpr int kMaxWinTiles = 256;
-
 // What a line of a group is: rows `row` and row + 1 of the batch
 struct InvLine {
     long long row;
@@ -382,7 +380,7 @@ k_rows_inv_pfa(const float2 *__restrict__ S, long long nrows, TileGeom g, int re
     constexpr int H = N / 2 + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int next;
-    __shared__ int cum[WIN ? kMaxWinTiles + 1 : 1];  // groups before tile t
+    __shared__ int cum[WIN ? MM_MAX_WIN_TILES + 1 : 1];  // groups before tile t
     __shared__ InvLine lines[2][kPfaNL];
     const PfaSmem<N> s = pfa_layout<N>(smem_raw, line_bytes<N>());
     float *rtab = reinterpret_cast<float *>(smem_raw + line_bytes<N>() + pfa_tail_bytes<N>());  // 1 / window count
