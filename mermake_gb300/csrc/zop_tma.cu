@@ -495,9 +495,6 @@ bool zth_split(int Z, int nt, int tt, int pb, ZthPlan *pl) {
 // 20 of Z = 56: 2.81 against 3.06) but for the depth with its own kernel (25
 // tiles of Z = 50: 4 frequencies 2.83, 8 2.94; 16 tiles 1.97 against 2.21).
 bool zth_plan(int Z, int nt, ZthPlan *pl) {
-#ifdef ZTH_FORCE
-    return zth_split(Z, nt, g_tt, g_pb, pl);
-#endif
     if (nt <= 2 && zth_split(Z, nt, nt, 16, pl) && pl->nchunks == 1) return true;
     if (nt <= 10) {
         double best = 0;
