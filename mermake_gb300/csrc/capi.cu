@@ -241,8 +241,8 @@ bool stitch_covers(const TileGeom &g) {
 // kept spots of a hyb tile have centroids inside it and read their maxima and
 // fit neighbourhoods, at most delta_fit + max(delta, delta_fit) closer to the
 // edge.
-// The z step of a batch: MM_ZFORM_REGISTERS (k_zth_apply over one shared
-// spectrum, else k_zpt_apply with a kernel per tile), _SHARED (k_zop_apply),
+// The z step of a batch: MM_ZFORM_REGISTERS (k_zfft_apply, else k_zth_apply over
+// one shared spectrum, else k_zpt_apply with a kernel per tile), _SHARED (k_zop_apply),
 // _DIRECT (k_zconv) or _TRANSFORMS (k_zpass).  The context's MM_OPT_ZFORM
 // choice when the batch qualifies for it (a z kernel, one spectrum for the
 // shared and tensor forms, the forms' shape limits), else the first of
@@ -259,6 +259,14 @@ bool zth_takes(const TileGeom &g, bool forced) {
     if (g.nt == 1 && !forced && mm_zpt_supported(g.Z, g.zpad, 1, plane)) return false;
     const int chunks = mm_zth_supported(g.Z, g.zpad, g.nt, plane);
     return chunks == 1 || (chunks > 1 && (forced || mm_zop_supported(g.Z, g.zpad) == 0));
+}
+
+// k_zfft_apply over one shared spectrum: from four tiles on it is the faster one
+// at every depth and padding it takes (1.0 to 1.8 times at P = 478 and 678, 26 <=
+// Z <= 56, 4 to 25 tiles; 3 tiles of Z = 50: 0.220 against 0.226 ms, of Z = 31
+// 0.140 against 0.128), its tables being made for two tiles as for many
+bool zfft_takes(const TileGeom &g, const float2 *zop) {
+    return g.npsf == 1 && g.nt >= 4 && mm_zfft_supported(g.Z, g.zpad, g.nt, (long long)g.P * g.H, zop) != 0;
 }
 
 int zform_of(const mm_ctx *c, const TileGeom &g, const float2 *zop) {
@@ -346,6 +354,10 @@ int run_tiles(mm_ctx *c, TileGeom g, const void *image, int dtype, const float *
         // the matrix applied on the tensor cores; the z kernel is read once per batch
         StageTimer t(c, ST_ZPASS, 2 * spec_b + 8.0 * wstride, st);
         if ((rc = mm_launch_zmma_apply(S, zop, g.Z, g.zpad, g.Zp, plane_c, g.nt, fresp, &sm->err, st))) return rc;
+    } else if (zform == MM_ZFORM_REGISTERS && zfft_takes(g, zop)) {
+        // by short transforms; the z kernel is read once per batch
+        StageTimer t(c, ST_ZPASS, 2 * spec_b + 8.0 * wstride, st);
+        if ((rc = mm_launch_zfft_apply(S, zop, g.Z, g.zpad, g.Zp, plane_c, g.nt, fresp, st))) return rc;
     } else if (zform == MM_ZFORM_REGISTERS && zth_takes(g, c->zform == MM_ZFORM_REGISTERS)) {
         // the matrix formed in registers, operands staged by TMA; the z kernel
         // is read once per batch

@@ -186,6 +186,11 @@ int mm_launch_zmma_apply(float2 *S, const float2 *w, int Z, int zpad, int Zp, lo
                          const float *fresp, unsigned *err, cudaStream_t st);
 int mm_launch_zth_apply(float2 *S, const float2 *w, int Z, int zpad, int Zp, long long plane, int nt,
                         const float *fresp, unsigned *err, cudaStream_t st);
+// The same for 26 <= Z <= 56 at zpad = Z - 1 or (Z - 2) / 2 by transforms of at
+// least 2 Z points in registers (zop_fft.cu).
+int mm_zfft_supported(int Z, int zpad, int nt, long long plane, const void *w);
+int mm_launch_zfft_apply(float2 *S, const float2 *w, int Z, int zpad, int Zp, long long plane, int nt,
+                         const float *fresp, cudaStream_t st);
 // The register form with a z kernel per tile (zop_pt.cu): tile t of the
 // launch, spectrum index t0 + t, takes the kernel w + (t0 + t) * wstride when
 // npsf > 1, else w.  Z a multiple of 5 up to 80, 1 <= zpad <= Z - 1, an even

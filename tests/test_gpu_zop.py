@@ -10,8 +10,8 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("ts,ov", [(14, 3), (30, 9)])  # planes of 2 and of 0 mod 8 frequencies
 def test_register_form_over_batch_sizes(Z, zpad, ts, ov):
     """Against the transforms over the padded depth (2e-5 of the largest voxel,
-    as for the other forms), and the same bits for every batch size: each
-    output sums its columns in the same order."""
+    as for the other forms).  Where the matrix forms take every batch, the same
+    bits for every batch size: each output sums its columns in the same order."""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from mermake_gb300 import _lib, deconvolver, synth
@@ -21,6 +21,7 @@ def test_register_form_over_batch_sizes(Z, zpad, ts, ov):
                                   beta=0.01)
     with _lib.zform(_lib.MM_ZFORM_TRANSFORMS):
         want = dec.apply(img, None)
+    transforms = 26 <= Z <= 56 and (zpad == Z - 1 or 2 * zpad == Z - 2)  # from four tiles on
     first = None
     with _lib.zform(_lib.MM_ZFORM_REGISTERS):
         for batch in (1, 2, 3, 4, 5, 6, 9, 11, 16):
@@ -28,6 +29,37 @@ def test_register_form_over_batch_sizes(Z, zpad, ts, ov):
             err = (got - want).abs().max() / want.abs().max()
             assert err < 2e-5, (batch, float(err))
             first = got if first is None else first
-            assert torch.equal(got, first), batch
+            assert transforms or torch.equal(got, first), batch
     # the library's own choice: one tile takes the per-tile form where it can
     assert torch.equal(dec.apply(img, None, batch=1), first)
+
+
+@pytest.mark.parametrize("Z", [25, 26, 30, 31, 35, 36, 40, 41, 45, 46, 50, 51, 56, 57])
+@pytest.mark.parametrize("near", [False, True])
+def test_short_transforms_at_the_edges_of_their_lengths(Z, near):
+    """The first and last depth of every length (and the depths beside them),
+    both paddings, planes that end inside a group of 64 frequencies, batches of
+    whole and of cut rounds, with and without the folded blur: against the
+    transforms over the padded depth, 2e-5 of the largest voxel as above.  A
+    tile's bits do not depend on its batch."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from mermake_gb300 import _lib, deconvolver, synth
+    if near and Z % 2:
+        pytest.skip("no such padding at an odd depth")
+    for ts, ov in ((14, 3), (30, 9)):
+        X, Y = 4 * ts - 1, 3 * ts
+        img = synth.hyb_stack(Z, X, Y, 40, seed=Z + ts).cuda()
+        dec = deconvolver.Deconvolver(synth.gaussian_psf((5, 7, 7), 1.2, 1.3), (Z, X, Y), tile_size=ts,
+                                      zpad=(Z - 2) // 2 if near else Z - 1, overlap=ov, beta=0.01)
+        for blur in (None, 6):
+            mode = _lib.MM_BLUR_EXACT if blur is None else _lib.MM_BLUR_SPECTRAL
+            got = {}
+            with _lib.blur_mode(mode):
+                with _lib.zform(_lib.MM_ZFORM_DIRECT):
+                    want = dec.apply(img, None, blur_radius=blur)
+                for batch in (4, 6, 12):
+                    got[batch] = dec.apply(img, None, blur_radius=blur, batch=batch)
+            err = (got[12] - want).abs().max() / want.abs().max()
+            assert err < 2e-5, (ts, blur, float(err))
+            assert torch.equal(got[4], got[12]) and torch.equal(got[6], got[12]), (ts, blur)
