@@ -28,7 +28,7 @@
 // What bounds it: instruction issue and fetch.  A column is about 7 k
 // instructions, nearly all straight-line code, 110 KB in all; warps that ran
 // through it apart (jobs taken from a counter, twelve warps) spent half of
-// their time waiting for instructions (3.4 ms).  So the two warps of an SM
+// their time waiting for instructions (3.4 ms at 25 tiles).  So the two warps of an SM
 // sub-partition run the same steps side by side, one of each half, and all
 // warps finish a group together.  At P = 678, Z = 50 (ms per launch, zpad 49 /
 // 24, the matrix form in brackets): 4 tiles 0.45 / 0.38 [0.55 / 0.58], 6 tiles
@@ -40,6 +40,8 @@
 // does not depend on the batch.  The largest error against 64-bit sums, over
 // random columns at Z = 50, was 5.3e-8 to 8.9e-8 of the largest output where
 // the matrix form has 4.7e-8 to 1.2e-7.
+#include <type_traits>
+
 #include "deconv.cuh"
 #include "fft_pfa.cuh"
 
@@ -287,43 +289,53 @@ k_zfft_apply(float2 *__restrict__ S, const float2 *__restrict__ w, const ZfArgs 
             float2 v[N], e0, e1;
             if (active) {
                 if (table) {
-                    const float sg = half ? -1.f : 1.f;
-                    if (kind == 0) {
+                    // g[s] + g[s + N] for the even half, g[s] - g[s + N] for the
+                    // odd one, g the generator: each warp of the pair loads one
+                    // part of it and hands over what the other needs (where
+                    // both loaded all of it a launch took 0.04 ms longer)
+                    constexpr int M0 = (N + 1) / 2;
+                    auto load = [&](auto odd) {
+                        constexpr int H = decltype(odd)::value, S0 = H ? M0 : 0, L = H ? N - M0 : M0;
+                        float2 lo[L], hi[L];
+                        auto in = [&](int s) { return s + N <= 2 * LO - 2 || (s + N <= 2 * N - 2 && s + N <= 2 * Z - 2); };
+                        if (kind == 0) {
 #pragma unroll
-                        for (int s = 0; s < N; ++s) {
-                            v[s] = s < LO || s < Z ? wrow(s) : make_float2(0.f, 0.f);
-                            if (N - s < LO || N - s < Z) {
-                                const float2 x = wrow(a.Zp - N + s);
-                                v[s] = make_float2(fmaf(sg, x.x, v[s].x), fmaf(sg, x.y, v[s].y));
+                            for (int i = 0; i < L; ++i) {
+                                const int s = S0 + i;
+                                lo[i] = s < LO || s < Z ? wrow(s) : make_float2(0.f, 0.f);
+                                hi[i] = N - s < LO || N - s < Z ? wrow(a.Zp - N + s) : make_float2(0.f, 0.f);
                             }
-                        }
-                    } else {
-                        // b[s + N], s + N <= 2 Z - 2, then b[s]; its second part
-                        // at zpad = Z - 1 only
+                        } else {
 #pragma unroll
-                        for (int s = 0; s < N; ++s) {
-                            v[s] = wrow(s);
-                            if (s + N <= 2 * N - 2) {
-                                const bool in = s + N <= 2 * LO - 2 || s + N <= 2 * Z - 2;
-                                const float2 x = wrow(s + N >= a.Zp ? s + N - a.Zp : s + N);
-                                v[s].x = fmaf(in ? sg : 0.f, x.x, v[s].x);
-                                v[s].y = fmaf(in ? sg : 0.f, x.y, v[s].y);
+                            for (int i = 0; i < L; ++i) {
+                                const int s = S0 + i;
+                                lo[i] = wrow(s);
+                                hi[i] = in(s) ? wrow(s + N >= a.Zp ? s + N - a.Zp : s + N) : make_float2(0.f, 0.f);
                             }
-                        }
-                        if (a.far) {
+                            if (a.far) {
 #pragma unroll
-                            for (int s = 0; s < N; ++s) {
-                                v[s] = padd(v[s], wrow(s + Z));
-                                if (s + N <= 2 * N - 2) {
-                                    const bool in = s + N <= 2 * LO - 2 || s + N <= 2 * Z - 2;
-                                    const int r = s + N + Z;
-                                    const float2 x = wrow(r >= a.Zp ? r - a.Zp : r);
-                                    v[s].x = fmaf(in ? sg : 0.f, x.x, v[s].x);
-                                    v[s].y = fmaf(in ? sg : 0.f, x.y, v[s].y);
+                                for (int i = 0; i < L; ++i) {
+                                    const int s = S0 + i, r = s + N + Z;
+                                    lo[i] = padd(lo[i], wrow(s + Z));
+                                    if (in(s)) hi[i] = padd(hi[i], wrow(r >= a.Zp ? r - a.Zp : r));
                                 }
                             }
                         }
-                    }
+#pragma unroll
+                        for (int i = 0; i < L; ++i) {
+                            const float2 sum = padd(lo[i], hi[i]), dif = psub(lo[i], hi[i]);
+                            v[S0 + i] = H ? dif : sum;
+                            buf[(S0 + i) * 32] = H ? sum : dif;
+                        }
+                        pair_sync(pair);
+                        constexpr int T0 = H ? 0 : M0;
+#pragma unroll
+                        for (int i = 0; i < N - L; ++i) v[T0 + i] = buf[(T0 + i) * 32];
+                    };
+                    if (half)
+                        load(std::true_type{});
+                    else
+                        load(std::false_type{});
                 } else {
                     cp_async_wait();
                     pair_sync(pair);
