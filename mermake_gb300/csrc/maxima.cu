@@ -169,46 +169,76 @@ constexpr int kMaxY1 = 8, kMaxY2 = 4;
 constexpr int kQueue = 32 * kMaxY1 + 32;
 static_assert(2 * 32 * kMaxY2 + 32 <= kQueue, "queue too small for the two-sign pass");
 constexpr int kNbBatch = 8;
+// Spheres of more than kManyNb neighbours: few voxels are above the nearest
+// kNear, and a lane that goes on through hundreds alone keeps its warp, so each
+// of those is tested by the whole warp, 32 neighbours side by side.  Radius 5
+// (514): both signs of a 50 x 1500 x 1302 DAPI block 0.59 -> 0.28 ms with its
+// fits, 21 k maxima of a 50 x 1024 x 1000 volume 0.85 -> 0.32; radius 3 (122)
+// 0.32 -> 0.19; radius 2 (32) gains nothing (1.6 M maxima 5.5 against 5.9 ms).
+constexpr int kManyNb = 64, kNear = 8;
+constexpr int kWarpBatch = 2;  // neighbours of a lane in flight there
 constexpr int kFitU = 2;  // fit sample rounds whose loads are in flight together (4 costs occupancy)
 
-// 1 when the voxel (raw value vr) is not below any in-range neighbour of
-// (z, x, y) in the sphere of radius delta, compared as transformed values.
-// The transform x -> x / div (div > 0, round to nearest) is monotone, so a
-// neighbour whose raw value is not above the voxel's (not below, for the
-// negated volume) cannot be above it after the transform either; only the
-// others are transformed and compared exactly.  An interior voxel (delta
-// from every face) reads its neighbours at fixed offsets, with no reflection.
-__device__ __forceinline__ bool max_test(const float *__restrict__ img, const Vols &V, Xform t, int Z, int X,
-                                         int Y, int z, int x, int y, float vr, const char4 *sph, int nn,
-                                         int delta) {
-    const float vt = xf(vr, t);
-    const bool mono = t.div >= 0.f;
-    const bool inner = z >= delta && z < Z - delta && x >= delta && x < X - delta && y >= delta && y < Y - delta;
-    const float *c = img + z * V.isz + x * V.isx + y;
+// A voxel (raw value vr) against its neighbours in the sphere of radius delta,
+// compared as transformed values.  The transform x -> x / div (div > 0, round
+// to nearest) is monotone, so a neighbour whose raw value is not above the
+// voxel's (not below, for the negated volume) cannot be above it after the
+// transform either; only the others are transformed and compared exactly.  An
+// interior voxel (delta from every face) reads its neighbours at fixed
+// offsets, with no reflection.
+struct MaxVoxel {
+    const float *img, *c;
+    const char4 *sph;
+    long long isz, isx;
+    int Z, X, Y, z, x, y;
+    float vr, vt;
+    Xform t;
+    bool inner;
+
+    __device__ __forceinline__ MaxVoxel(const float *img_, const Vols &V, Xform t_, int Z_, int X_, int Y_, unsigned key,
+                                        int y_, float vr_, const char4 *sph_, int delta)
+        : img(img_), sph(sph_), isz(V.isz), isx(V.isx), Z(Z_), X(X_), Y(Y_), z((int)(key & 0xffffu)),
+          x((int)(key >> 16)), y(y_), vr(vr_), t(t_) {
+        vt = xf(vr, t);
+        inner = z >= delta && z < Z - delta && x >= delta && x < X - delta && y >= delta && y < Y - delta;
+        c = img + z * isz + x * isx + y;
+    }
+    // neighbour q's raw value, NaN (never above) where there is none
+    __device__ __forceinline__ float at(int q) const {
+        const char4 o = sph[q];
+        if (inner) return c[o.x * isz + o.y * isx + o.z];
+        const int nz = refl(z + o.x, Z), nx = refl(x + o.y, X), ny = refl(y + o.z, Y);
+        return nz >= 0 && nz < Z && nx >= 0 && nx < X && ny >= 0 && ny < Y ? img[nz * isz + nx * isx + ny] : NAN;
+    }
+    __device__ __forceinline__ bool below(float nb) const {
+        const bool may = t.neg ? nb < vr : nb > vr;
+        return (!(t.div >= 0.f) || may) && vt < xf(nb, t);
+    }
+};
+
+// 1 when the voxel is not below any of its first nn neighbours (a lane per voxel)
+__device__ __forceinline__ bool max_test(const MaxVoxel &m, int nn) {
     for (int q0 = 0; q0 < nn; q0 += kNbBatch) {
         float nb[kNbBatch];
 #pragma unroll
-        for (int u = 0; u < kNbBatch; ++u) {
-            nb[u] = NAN;  // no neighbour: never above
-            const int q = q0 + u;
-            if (q < nn) {
-                const char4 o = sph[q];
-                if (inner) {
-                    nb[u] = c[o.x * V.isz + o.y * V.isx + o.z];
-                } else {
-                    const int nz = refl(z + o.x, Z), nx = refl(x + o.y, X), ny = refl(y + o.z, Y);
-                    if (nz >= 0 && nz < Z && nx >= 0 && nx < X && ny >= 0 && ny < Y)
-                        nb[u] = img[nz * V.isz + nx * V.isx + ny];
-                }
-            }
-        }
+        for (int u = 0; u < kNbBatch; ++u) nb[u] = q0 + u < nn ? m.at(q0 + u) : NAN;
         bool below = false;
 #pragma unroll
-        for (int u = 0; u < kNbBatch; ++u) {
-            const bool may = t.neg ? nb[u] < vr : nb[u] > vr;
-            if (!mono || may) below |= vt < xf(nb[u], t);
-        }
+        for (int u = 0; u < kNbBatch; ++u) below |= m.below(nb[u]);
         if (below) return false;
+    }
+    return true;
+}
+// the same of one voxel's neighbours [q0, nn), the warp's lanes side by side
+__device__ __forceinline__ bool max_test_warp(const MaxVoxel &m, int q0, int nn, int lane) {
+    for (; q0 < nn; q0 += 32 * kWarpBatch) {
+        float nb[kWarpBatch];
+#pragma unroll
+        for (int u = 0; u < kWarpBatch; ++u) nb[u] = q0 + 32 * u + lane < nn ? m.at(q0 + 32 * u + lane) : NAN;
+        bool below = false;
+#pragma unroll
+        for (int u = 0; u < kWarpBatch; ++u) below |= m.below(nb[u]);
+        if (__any_sync(0xffffffffu, below)) return false;
     }
     return true;
 }
@@ -234,18 +264,23 @@ __device__ __forceinline__ void test_round(const float *__restrict__ img, const 
                                            const float *vq, int cnt, unsigned lane, int vi, uint2 *__restrict__ cand,
                                            unsigned cap, unsigned *__restrict__ count, uint2 *__restrict__ cand2,
                                            unsigned *__restrict__ count2, bool both) {
-    bool is_max = false, neg = false;
-    unsigned key = 0;
-    int y = 0;
-    if ((int)lane < cnt) {
-        key = k[lane];
-        const int e = yq[lane];
-        neg = (e >> 30) & 1;
-        y = e & 0x3fffffff;
+    const bool mine = (int)lane < cnt;
+    const unsigned key = mine ? k[lane] : 0;
+    const int e = mine ? yq[lane] : 0, y = e & 0x3fffffff;
+    const bool neg = (e >> 30) & 1;
+    auto voxel = [&](unsigned kl, int el, float vl) {
         Xform ts = t;
-        if (neg) ts.neg = !ts.neg;
-        is_max = max_test(img, V, ts, Z, X, Y, (int)(key & 0xffffu), (int)(key >> 16), y, vq[lane], sph, nn, delta);
-    }
+        if ((el >> 30) & 1) ts.neg = !ts.neg;
+        return MaxVoxel(img, V, ts, Z, X, Y, kl, el & 0x3fffffff, vl, sph, delta);
+    };
+    const int near = nn > kManyNb ? kNear : nn;
+    bool is_max = mine && max_test(voxel(key, e, vq[lane]), near);
+    if (near < nn)
+        for (unsigned left = __ballot_sync(0xffffffffu, is_max); left; left &= left - 1) {
+            const int l = __ffs(left) - 1;
+            const bool m = max_test_warp(voxel(k[l], yq[l], vq[l]), near, nn, (int)lane);
+            if ((int)lane == l) is_max = m;
+        }
     append_cand(is_max && !neg, key, y, vi, lane, cand, cap, count);
     if (both) append_cand(is_max && neg, key, y, vi, lane, cand2, cap, count2);
 }

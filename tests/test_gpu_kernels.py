@@ -286,6 +286,26 @@ def test_maxima_chunks_without_a_candidate(mm, neg, div, th):
     assert bool(torch.isnan(with_nan[:, 7]).any())
 
 
+@pytest.mark.parametrize("delta", [2, 3, 4, 5])  # a lane per voxel up to 2, then the warp per voxel
+@pytest.mark.parametrize("neg,div", [(False, 0.0), (True, 0.0), (False, 3.0), (True, 3.0)])
+def test_maxima_of_wide_spheres_with_ties(mm, delta, neg, div):
+    """Smooth volumes of few levels (plateaus: equal neighbours keep both
+    voxels), dimensions below and above the sphere's: the oracle's maxima."""
+    rng = np.random.default_rng(delta)
+    for shape in ((6, 9, 40), (13, 21, 67)):
+        im = rng.normal(0, 1, shape)
+        for ax in range(3):
+            im = im + np.roll(im, 1, ax) + np.roll(im, -1, ax)
+        im = np.round(im / 2).astype(np.float32)
+        got = mm["maxima"].find_local_maxima(torch.from_numpy(im).cuda(), 0.5, delta, 1, norm_div=div,
+                                             negate=neg).cpu().numpy()
+        v = im / np.float32(div) if div else im
+        v = -v if neg else v
+        want = ck.find_local_maxima(np.ascontiguousarray(v), 0.5, delta, 1, im, 1.0, 1.5)
+        assert len(want) > 3
+        assert_rows_close(got, want)
+
+
 def test_subtract_u16(mm):
     rng = np.random.default_rng(2)
     x = rng.integers(0, 65536, (4, 7, 9)).astype(np.uint16)
