@@ -300,12 +300,12 @@ def job_rate(world, units_per_rank, steps, total_ms):
 
 
 def zpass_flops(w, s, zform="auto"):
-    """FP32 flops of one FOV's z passes, by the form each channel's batch runs
-    (the library's choice in run_tiles): one Z x Z complex matrix per frequency
-    and tile when one spectrum serves a batch of >= 10 tiles of height <= 64,
-    or when each tile's matrix is formed from its own z kernel (Z a multiple
-    of 5 up to 80, 1 <= zpad <= Z - 1); else the direct sum over the padded
-    planes (outputs and planes in blocks of 8).  A complex FMA is 8 flops."""
+    """FP32 flops of one FOV's z passes done as sums: one Z x Z complex matrix per
+    frequency and tile when one spectrum serves a batch of >= 10 tiles of
+    height <= 64, or when each tile's matrix is formed from its own z kernel (Z
+    a multiple of 5 up to 80, 1 <= zpad <= Z - 1); else the direct sum over the
+    padded planes (outputs and planes in blocks of 8).  A complex FMA is 8
+    flops."""
     shape = (w["Z"], w["X"], w["Y"])
     out = 0.0
     for dec, n in ((s["dec_h"], w["colours"]), (s["dec_d"], 1 if s["dec_d"] is not None else 0)):
@@ -321,6 +321,31 @@ def zpass_flops(w, s, zform="auto"):
         else:
             per = -(-Z // 8) * 8 * (-(-dec.Zp // 8) * 8)
         out += n * nt * plane * per * 8.0
+    return out
+
+
+def zpass_run_flops(w, s, zform="auto"):
+    """FP32 flops that one FOV's z passes run: zpass_flops, but for channels
+    that the library's choice takes through transforms in registers (one
+    spectrum, at least 4 tiles, 26 <= Z <= 56, zpad Z - 1 or (Z - 2) / 2).
+    There a column takes four transforms of N points (5 N log2 N flops each),
+    two products per frequency of 2 N, the odd frequencies' two twiddles a
+    point and, at zpad = Z - 1, two end terms a plane."""
+    import math
+    out = zpass_flops(w, s, zform)
+    if zform not in ("auto", "registers"):
+        return out
+    shape = (w["Z"], w["X"], w["Y"])
+    for dec, n in ((s["dec_h"], w["colours"]), (s["dec_d"], 1 if s["dec_d"] is not None else 0)):
+        if not n or dec.z_operator is None or dec.psf_fft.shape[0] != 1:
+            continue
+        nt, Z = dec.n_tiles(shape), dec.tile_height
+        if nt < 4 or not 26 <= Z <= 56 or dec.zpad not in (Z - 1, (Z - 2) / 2):
+            continue
+        N = next(k for k in (30, 35, 40, 45, 50, 56) if Z <= k)
+        per = 4 * 5 * N * math.log2(N) + 2 * N * 16 + 2 * N * 8 + (Z * 16 if dec.zpad == Z - 1 else 0)
+        one = dict(s, dec_h=dec, dec_d=None)
+        out += n * nt * dec.P * dec.H * per - zpass_flops(dict(w, colours=n), one, zform)
     return out
 
 
@@ -456,14 +481,14 @@ def gpu_arm(args, rank, world, local):
         "clocks": clk.summary(),
     }
     if dom == "zpass" and args.form == "batched":
-        # the z pass is bound by FP32 FMA issue, not by bytes: the line's bound
+        # the z pass is bound by FP32 issue, not by bytes: the line's bound
         # is its arithmetic against the nominal FP32 peak (SMs x 128 lanes x 2
         # flops x the sampled maximum SM clock; the measured peaks file has no
         # FP32 figure), with the HBM figures beside it
         props = torch.cuda.get_device_properties(dev)
         mhz = (line["clocks"] or {}).get("sm_max_mhz") or peaks.get("sm_max_mhz") or 2070.0
         fpeak = props.multi_processor_count * 128 * 2 * mhz * 1e6 / 1e12
-        fl = zpass_flops(w, s, args.zform) * args.steps / dl
+        fl = zpass_run_flops(w, s, args.zform) * args.steps / dl
         fach = fl / ((dms / dl) / 1e3) / 1e12
         rf = line["roofline"]
         hbm = {k: rf[k] for k in ("achieved", "peak", "unit", "frac", "peak_source")}

@@ -82,12 +82,13 @@ enum { MM_BLUR_AUTO = 0, MM_BLUR_EXACT = 1, MM_BLUR_SPECTRAL = 2 };
 /* MM_OPT_ZFORM selects how the z step of tile_wise (padding by reflection,
  * transforms over Zp, times W, crop; mermake/deconvolver.py:139-157) runs:
  *   MM_ZFORM_AUTO (default): the first form below that the batch qualifies for
- *     (over one shared spectrum, the matrix forms from batches of 10 tiles);
- *   MM_ZFORM_REGISTERS: one Z x Z matrix per frequency, formed in registers
- *     from the z kernel (Z a multiple of 5, 1 <= zpad <= Z - 1): over one
- *     spectrum shared by the batch, operands staged by TMA; or, with a
- *     spectrum per tile or a batch below 10 tiles, each tile's matrix from its
- *     own z kernel (Z <= 80);
+ *     (the shared-memory matrix from batches of 10 tiles);
+ *   MM_ZFORM_REGISTERS: in registers from the z kernel, 1 <= zpad <= Z - 1.
+ *     Over one spectrum shared by the batch: by transforms of 2 Z points and
+ *     more (at least 4 tiles, 26 <= Z <= 56, zpad Z - 1 or (Z - 2) / 2), else
+ *     one Z x Z matrix per frequency, operands staged by TMA.  With a spectrum
+ *     per tile: each tile's matrix from its own z kernel (Z a multiple of 5,
+ *     Z <= 80);
  *   MM_ZFORM_SHARED: the same matrix summed into shared memory (one spectrum,
  *     Z <= 64, at most four copies of a plane);
  *   MM_ZFORM_DIRECT: the direct sum over the padded planes per tile;
@@ -150,7 +151,7 @@ int mm_wiener_spectrum(mm_ctx *ctx, const float *psf, int pz, int px, int py, in
  * sum_z zop[(zpad + i - z) mod Zp] x[map(z)] per frequency.  Passing zop
  * (one kernel per spectrum, laid out like W) to mm_deconv_tiles /
  * mm_hyb_spots / mm_dapi_spots replaces the two padded-depth transforms of
- * each tile: with one spectrum and batches of at least 10 tiles by one Z x Z
+ * each tile: with one spectrum by transforms in registers or by one Z x Z
  * complex matrix per frequency over the batch (each entry a sum of at most
  * four kernel samples; tile_height <= 64 and no plane copied more than four
  * times by the padding), otherwise by that sum taken directly per tile

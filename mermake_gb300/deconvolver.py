@@ -111,8 +111,8 @@ class Deconvolver:
     # Zp, times the spectrum, crop) is, per (x, y) frequency, a sum over the
     # padded planes weighted by the inverse DFT of the spectrum along z
     # (csrc/zop.cu).  One kernel per spectrum, the size of psf_fft, kept
-    # beside it.  With one PSF and batches of >= 10 tiles the sum runs as a
-    # Z x Z matrix per frequency over the batch; otherwise directly per tile.
+    # beside it.  The sum runs by transforms or as a Z x Z matrix per frequency,
+    # over a batch of tiles with one PSF and per tile with several.
     def _want_z_operator(self, request):
         ok = bool(self.tile_size) and bool(_lib.lib().mm_zkernel_supported(self.tile_height, self.zpad))
         if request is True and not ok:

@@ -11,15 +11,16 @@ time).  ``default_batch`` therefore takes all tiles, up to a scratch budget
 (``SCRATCH_BYTES``), and the library picks the z form (``MM_ZFORM_AUTO``).
 
 ``autotune`` times, on a real channel, every candidate batch size with every
-z form the geometry qualifies for (the matrix in registers, over one shared
-spectrum or per tile, the matrix on the tensor cores or in shared memory, the
-direct sum per tile, the transforms over the padded depth;
+z form the geometry qualifies for (in registers, over one shared spectrum or
+per tile, the matrix on the tensor cores or in shared memory, the direct sum
+per tile, the transforms over the padded depth;
 ``mm_ctx_set_option(MM_OPT_ZFORM)``) and keeps the fastest pair on the
 Deconvolver, where the drivers find it (``settings_for``).
 
 With several PSFs every batch size gives the same rows.  The z forms, and
-with one PSF batches on either side of the matrix forms' 10 tiles, give the
-same voxels within float32 rounding (about 1e-7 relative), which can move a
+with one PSF batches on either side of 4 tiles (from where the register form
+works by transforms at common depths), give the same voxels within float32
+rounding (about 1e-7 relative), which can move a
 spot that sits on the threshold.
 """
 from __future__ import annotations
