@@ -3,6 +3,7 @@
 //   box_1d       blur.cu:1-52       truncated-window mean along one axis (any layout)
 //   subtract     math.py:4-33       uint16 saturating / reflecting subtraction
 //   sumsq        __main__.py:221    sum of squares for the DAPI RMS (double accumulation)
+#include <float.h>
 #include <stdint.h>
 #include "deconv.cuh"
 
@@ -144,7 +145,36 @@ __global__ void k_sumsq(const float *__restrict__ x, long long n, double *__rest
     if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
         const float4 *x4 = reinterpret_cast<const float4 *>(x);
         const long long n4 = n / 4;
-        for (long long i = tid; i < n4; i += nth) {
+        // Conversions to double and additions there bounded the pass at one each
+        // per four values (0.103 ms at any grid).  Now four groups of four
+        // squares are added without loss, as a float and what its rounding left
+        // (two-sum, Knuth), and the left-overs, 2^-24 of the sums, collect in a
+        // float.  50 x 1500 x 1302 voxels: the DAPI block's stage 0.123 -> 0.080
+        // ms at four CTAs an SM (eight 0.09)
+        long long i = tid;
+        float rest = 0.f;
+        bool fine = true;
+        for (; i + 3 * nth < n4; i += 4 * nth) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = x4[i + u * nth];
+            float s = 0.f;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float q = fmaf(v[u].w, v[u].w, fmaf(v[u].z, v[u].z, fmaf(v[u].y, v[u].y, v[u].x * v[u].x)));
+                const float t = __fadd_rn(s, q), z = __fsub_rn(t, s);
+                rest = __fadd_rn(rest, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(q, z)));
+                s = t;
+            }
+            fine &= s <= FLT_MAX;
+            acc += (double)s;
+        }
+        acc += (double)rest;
+        if (!fine) {  // a sum without a remainder (infinite, NaN): group by group in double
+            acc = 0.0;
+            i = tid;
+        }
+        for (; i < n4; i += nth) {
             const float4 v = x4[i];
             acc += (double)fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x)));
         }
@@ -274,7 +304,9 @@ int mm_launch_sumsq(const float *x, long long n, double *parts, double *out, cud
         MM_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(double), st));
         return MM_OK;
     }
-    const int g = grid_for(n);
+    // 16 values and more a thread, four CTAs an SM
+    int g = grid_for((n + 15) / 16);
+    if (g > 152 * 4) g = 152 * 4;
     k_sumsq<<<g, 256, 0, st>>>(x, n, parts);
     MM_CHECK_LAUNCH();
     return mm_launch_sum_parts(parts, g, out, st);

@@ -39,3 +39,19 @@ def test_apply_and_dapi_buffer_match_the_oracle_where_tiles_write(X, Y, ts, ov, 
     got = buf.cpu().numpy()
     assert np.abs(got[there] - want[there]).max() < 1e-5 * np.abs(want[there]).max()
     assert np.all(got[~there] == 0.0)
+
+
+@pytest.mark.parametrize("Z,X,Y", [(2, 40, 40), (5, 80, 77), (7, 123, 131), (30, 300, 256)])
+def test_dapi_rms_over_whole_and_cut_rounds_of_the_sum(Z, X, Y):
+    """The divisor is the root of a sum of squares accumulated beyond float32,
+    rounded to float32 three times: 2e-7 of it."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from mermake_gb300 import deconvolver, pipeline, synth
+    img = synth.dapi_stack(Z, X, Y, seed=X, n_nuclei=6)
+    dec = deconvolver.Deconvolver(synth.gaussian_psf((5, 7, 7), 1.2, 1.3), (Z, X, Y), tile_size=40, zpad=1, overlap=9,
+                                  beta=0.01)
+    _, _, buf, rms = pipeline.dapi_spots(dec, img.cuda(), None, threshold=3.0, delta=1, delta_fit=1)
+    v = buf.cpu().numpy().astype(np.float64)
+    want = np.sqrt((v * v).sum() / v.size)
+    assert abs(rms - want) <= 2e-7 * want
