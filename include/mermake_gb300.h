@@ -88,7 +88,7 @@ enum { MM_BLUR_AUTO = 0, MM_BLUR_EXACT = 1, MM_BLUR_SPECTRAL = 2 };
  *     more (at least 4 tiles, 26 <= Z <= 56, zpad Z - 1 or (Z - 2) / 2), else
  *     one Z x Z matrix per frequency, operands staged by TMA.  With a spectrum
  *     per tile: each tile's matrix from its own z kernel (Z a multiple of 5,
- *     Z <= 80);
+ *     Z <= 80), else the transforms;
  *   MM_ZFORM_SHARED: the same matrix summed into shared memory (one spectrum,
  *     Z <= 64, at most four copies of a plane);
  *   MM_ZFORM_DIRECT: the direct sum over the padded planes per tile;

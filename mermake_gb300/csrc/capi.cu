@@ -242,7 +242,7 @@ bool stitch_covers(const TileGeom &g) {
 // fit neighbourhoods, at most delta_fit + max(delta, delta_fit) closer to the
 // edge.
 // The z step of a batch: MM_ZFORM_REGISTERS (k_zfft_apply, else k_zth_apply over
-// one shared spectrum, else k_zpt_apply with a kernel per tile), _SHARED (k_zop_apply),
+// one shared spectrum, else k_zpt_apply or k_zfft_tiles with a kernel per tile), _SHARED (k_zop_apply),
 // _DIRECT (k_zconv) or _TRANSFORMS (k_zpass).  The context's MM_OPT_ZFORM
 // choice when the batch qualifies for it (a z kernel, one spectrum for the
 // shared and tensor forms, the forms' shape limits), else the first of
@@ -269,6 +269,17 @@ bool zfft_takes(const TileGeom &g, const float2 *zop) {
     return g.npsf == 1 && g.nt >= 4 && mm_zfft_supported(g.Z, g.zpad, g.nt, (long long)g.P * g.H, zop) != 0;
 }
 
+// k_zfft_tiles, a z kernel per tile, at depths that k_zpt_apply does not take: 16
+// tiles of 300 at Z = 37 1.16 ms against the direct sum's 1.89, at Z = 48 2.03
+// against 2.78, 25 tiles of 200 at Z = 27 0.74 against 1.09.  Where k_zpt_apply
+// takes the depth it is the faster one at zpad = Z - 1 (Z = 40 1.68 against 2.45 for
+// 32 tiles, Z = 45 1.49 against 1.56 for 16)
+bool zfft_tiles_takes(const TileGeom &g, const float2 *zop) {
+    const long long plane = (long long)g.P * g.H;
+    return g.npsf > 1 && !mm_zpt_supported(g.Z, g.zpad, g.nt, plane) &&
+           mm_zfft_supported(g.Z, g.zpad, g.nt, plane, zop) != 0;
+}
+
 int zform_of(const mm_ctx *c, const TileGeom &g, const float2 *zop) {
     const long long plane = (long long)g.P * g.H;
     // forced: the context's own choice, which takes any batch the form takes
@@ -281,7 +292,7 @@ int zform_of(const mm_ctx *c, const TileGeom &g, const float2 *zop) {
                 // per-tile form only where k_zth_apply does not take it
                 if (zth_takes(g, forced)) return true;
                 if (g.npsf == 1 && g.nt >= min_tiles && mm_zop_supported(g.Z, g.zpad) != 0) return false;
-                return mm_zpt_supported(g.Z, g.zpad, g.nt, plane) != 0;
+                return mm_zpt_supported(g.Z, g.zpad, g.nt, plane) != 0 || zfft_tiles_takes(g, zop);
             }
             case MM_ZFORM_SHARED:
                 return zop && g.npsf == 1 && g.nt >= min_tiles && mm_zop_supported(g.Z, g.zpad) != 0;
@@ -363,6 +374,11 @@ int run_tiles(mm_ctx *c, TileGeom g, const void *image, int dtype, const float *
         // is read once per batch
         StageTimer t(c, ST_ZPASS, 2 * spec_b + 8.0 * wstride, st);
         if ((rc = mm_launch_zth_apply(S, zop, g.Z, g.zpad, g.Zp, plane_c, g.nt, fresp, &sm->err, st))) return rc;
+    } else if (zform == MM_ZFORM_REGISTERS && zfft_tiles_takes(g, zop)) {
+        // by short transforms with each tile's own z kernel, read once per tile
+        StageTimer t(c, ST_ZPASS, 2 * spec_b + w_b, st);
+        if ((rc = mm_launch_zfft_tiles(S, zop, wstride, g.Z, g.zpad, g.Zp, plane_c, g.t0, g.nt, g.npsf, fresp, st)))
+            return rc;
     } else if (zform == MM_ZFORM_REGISTERS) {
         // the same with each tile's own z kernel, read once per tile
         StageTimer t(c, ST_ZPASS, 2 * spec_b + (g.npsf == 1 ? 8.0 * wstride : w_b), st);

@@ -191,6 +191,10 @@ int mm_launch_zth_apply(float2 *S, const float2 *w, int Z, int zpad, int Zp, lon
 int mm_zfft_supported(int Z, int zpad, int nt, long long plane, const void *w);
 int mm_launch_zfft_apply(float2 *S, const float2 *w, int Z, int zpad, int Zp, long long plane, int nt,
                          const float *fresp, cudaStream_t st);
+// The same with a z kernel per tile: tile t of the launch, spectrum index t0 + t,
+// takes w + (t0 + t) * wstride when npsf > 1, else w.
+int mm_launch_zfft_tiles(float2 *S, const float2 *w, long long wstride, int Z, int zpad, int Zp, long long plane, int t0,
+                         int nt, int npsf, const float *fresp, cudaStream_t st);
 // The register form with a z kernel per tile (zop_pt.cu): tile t of the
 // launch, spectrum index t0 + t, takes the kernel w + (t0 + t) * wstride when
 // npsf > 1, else w.  Z a multiple of 5 up to 80, 1 <= zpad <= Z - 1, an even

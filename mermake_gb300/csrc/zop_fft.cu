@@ -222,16 +222,15 @@ constexpr size_t zf_buffer(int n) { return sizeof(float2) * n * 32; }  // exchan
 // p: even frequencies 2p (H false) have q = -p, odd ones 2p + 1 q = -p - 1.
 // Real and imaginary parts change places, so that the forward transform that
 // follows is the inverse with its parts in each other's place.
-template <int N, bool H>
-__device__ __forceinline__ void zf_mix(float2 *v, const float2 *tab) {
-    const float2 *A = tab + (H ? 2 * N * kPB : 0), *B = A + N * kPB;
+template <int N, bool H, int PB>
+__device__ __forceinline__ void zf_mix(float2 *v, const float2 *A, const float2 *B) {
 #pragma unroll
     for (int p = 0; p < N; ++p) {
         const int q = H ? N - 1 - p : (N - p) % N;
         if (q < p) continue;
         const float2 xp = v[p], xq = v[q];
         auto make = [&](int k, float2 x, float2 y) {
-            const float2 a = A[k * kPB], b = B[k * kPB];
+            const float2 a = A[k * PB], b = B[k * PB];
             float2 r = make_float2(a.x * x.x, a.x * x.y);
             r.x = fmaf(-a.y, x.y, r.x);
             r.y = fmaf(a.y, x.x, r.y);
@@ -244,6 +243,61 @@ __device__ __forceinline__ void zf_mix(float2 *v, const float2 *tab) {
         v[p] = make(p, xp, xq);
         if (q != p) v[q] = make(q, xq, xp);
     }
+}
+
+// The N values whose transform is one half (even or odd) of the frequencies of
+// the generator a (kind 0) or b (kind 1): g[s] + g[s + N] for the even half, g[s]
+// - g[s + N] for the odd one.  Each warp of the pair loads one part of it and
+// hands over what the other needs (where both loaded all of it a launch took
+// 0.04 ms longer).
+template <int N>
+__device__ __forceinline__ void zf_generator(float2 *v, int kind, int half, const char *wp, unsigned pb8, const ZfArgs &a,
+                                             float2 *buf, int pair) {
+    constexpr int LO = zf_low(N), M0 = (N + 1) / 2;
+    const int Z = a.Z;
+    auto wrow = [&](int row) { return __ldg(reinterpret_cast<const float2 *>(wp + (unsigned)row * pb8)); };
+    auto load = [&](auto odd) {
+        constexpr int H = decltype(odd)::value, S0 = H ? M0 : 0, L = H ? N - M0 : M0;
+        float2 lo[L], hi[L];
+        auto in = [&](int s) { return s + N <= 2 * LO - 2 || (s + N <= 2 * N - 2 && s + N <= 2 * Z - 2); };
+        if (kind == 0) {
+#pragma unroll
+            for (int i = 0; i < L; ++i) {
+                const int s = S0 + i;
+                lo[i] = s < LO || s < Z ? wrow(s) : make_float2(0.f, 0.f);
+                hi[i] = N - s < LO || N - s < Z ? wrow(a.Zp - N + s) : make_float2(0.f, 0.f);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < L; ++i) {
+                const int s = S0 + i;
+                lo[i] = wrow(s);
+                hi[i] = in(s) ? wrow(s + N >= a.Zp ? s + N - a.Zp : s + N) : make_float2(0.f, 0.f);
+            }
+            if (a.far) {
+#pragma unroll
+                for (int i = 0; i < L; ++i) {
+                    const int s = S0 + i, r = s + N + Z;
+                    lo[i] = padd(lo[i], wrow(s + Z));
+                    if (in(s)) hi[i] = padd(hi[i], wrow(r >= a.Zp ? r - a.Zp : r));
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < L; ++i) {
+            const float2 sum = padd(lo[i], hi[i]), dif = psub(lo[i], hi[i]);
+            v[S0 + i] = H ? dif : sum;
+            buf[(S0 + i) * 32] = H ? sum : dif;
+        }
+        pair_sync(pair);
+        constexpr int T0 = H ? 0 : M0;
+#pragma unroll
+        for (int i = 0; i < N - L; ++i) v[T0 + i] = buf[(T0 + i) * 32];
+    };
+    if (half)
+        load(std::true_type{});
+    else
+        load(std::false_type{});
 }
 
 template <int N>
@@ -289,53 +343,7 @@ k_zfft_apply(float2 *__restrict__ S, const float2 *__restrict__ w, const ZfArgs 
             float2 v[N], e0, e1;
             if (active) {
                 if (table) {
-                    // g[s] + g[s + N] for the even half, g[s] - g[s + N] for the
-                    // odd one, g the generator: each warp of the pair loads one
-                    // part of it and hands over what the other needs (where
-                    // both loaded all of it a launch took 0.04 ms longer)
-                    constexpr int M0 = (N + 1) / 2;
-                    auto load = [&](auto odd) {
-                        constexpr int H = decltype(odd)::value, S0 = H ? M0 : 0, L = H ? N - M0 : M0;
-                        float2 lo[L], hi[L];
-                        auto in = [&](int s) { return s + N <= 2 * LO - 2 || (s + N <= 2 * N - 2 && s + N <= 2 * Z - 2); };
-                        if (kind == 0) {
-#pragma unroll
-                            for (int i = 0; i < L; ++i) {
-                                const int s = S0 + i;
-                                lo[i] = s < LO || s < Z ? wrow(s) : make_float2(0.f, 0.f);
-                                hi[i] = N - s < LO || N - s < Z ? wrow(a.Zp - N + s) : make_float2(0.f, 0.f);
-                            }
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < L; ++i) {
-                                const int s = S0 + i;
-                                lo[i] = wrow(s);
-                                hi[i] = in(s) ? wrow(s + N >= a.Zp ? s + N - a.Zp : s + N) : make_float2(0.f, 0.f);
-                            }
-                            if (a.far) {
-#pragma unroll
-                                for (int i = 0; i < L; ++i) {
-                                    const int s = S0 + i, r = s + N + Z;
-                                    lo[i] = padd(lo[i], wrow(s + Z));
-                                    if (in(s)) hi[i] = padd(hi[i], wrow(r >= a.Zp ? r - a.Zp : r));
-                                }
-                            }
-                        }
-#pragma unroll
-                        for (int i = 0; i < L; ++i) {
-                            const float2 sum = padd(lo[i], hi[i]), dif = psub(lo[i], hi[i]);
-                            v[S0 + i] = H ? dif : sum;
-                            buf[(S0 + i) * 32] = H ? sum : dif;
-                        }
-                        pair_sync(pair);
-                        constexpr int T0 = H ? 0 : M0;
-#pragma unroll
-                        for (int i = 0; i < N - L; ++i) v[T0 + i] = buf[(T0 + i) * 32];
-                    };
-                    if (half)
-                        load(std::true_type{});
-                    else
-                        load(std::false_type{});
+                    zf_generator<N>(v, kind, half, wp, pb8, a, buf, pair);
                 } else {
                     cp_async_wait();
                     pair_sync(pair);
@@ -360,9 +368,9 @@ k_zfft_apply(float2 *__restrict__ S, const float2 *__restrict__ w, const ZfArgs 
                     zdft<N, false>(v);
                     if (table || dir) break;
                     if (half)
-                        zf_mix<N, true>(v, tab);
+                        zf_mix<N, true, kPB>(v, tab + 2 * N * kPB, tab + 3 * N * kPB);
                     else
-                        zf_mix<N, false>(v, tab);
+                        zf_mix<N, false, kPB>(v, tab, tab + N * kPB);
                 }
             }
             if (table) {
@@ -433,6 +441,136 @@ k_zfft_apply(float2 *__restrict__ S, const float2 *__restrict__ w, const ZfArgs 
     }
 }
 
+// ---------------------------------------------------------------------------
+// A z kernel per tile (or few tiles): the pair of warps makes its own tables.  An
+// item is a tile and 32 frequencies; a warp does its half of both generators, of
+// the planes and of the inverse one after the other, with its tables in its own
+// rows of shared memory.  The CTA's pairs start their items together (see above).
+// Bound like the other kernel, with the loads of the z kernel exposed besides: 16
+// tiles of 300 at Z = 37 take 1.16 ms (1.89 with the direct sum; their 3.0 GB a
+// copy's 0.45).
+// ---------------------------------------------------------------------------
+constexpr size_t zt_warp(int n) { return sizeof(float2) * 2 * n * 32; }
+constexpr int zt_warps(int n) { return n <= 45 ? 8 : 6; }
+constexpr size_t zt_smem(int n) { return zt_warps(n) * zt_warp(n) + zt_warps(n) / 2 * zf_buffer(n); }
+
+template <int N>
+__global__ void __launch_bounds__(zt_warps(N) * 32, 1)
+k_zfft_tiles(float2 *__restrict__ S, const float2 *__restrict__ w, long long wstride, int t0, int npsf, const ZfArgs a) {
+    constexpr int LO = zf_low(N), W = zt_warps(N), NP = W / 2;
+    extern __shared__ __align__(16) unsigned char zf_smem[];
+    const int Z = a.Z, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int half = warp / NP, pair = warp % NP;
+    float2 *tab = reinterpret_cast<float2 *>(zf_smem + warp * zt_warp(N)) + lane;
+    float2 *xbuf = reinterpret_cast<float2 *>(zf_smem + W * zt_warp(N)) + pair * N * 32, *buf = xbuf + lane;
+    const unsigned pb8 = (unsigned)a.plane * 8u;  // bytes of a plane (checked by the launcher)
+    const long long total = (long long)a.ngroups * a.nt;
+    for (long long first = (long long)blockIdx.x * NP; first < total; first += (long long)gridDim.x * NP) {
+        __syncthreads();
+        const long long item = first + pair;
+        if (item >= total) continue;
+        const int t = (int)(item / a.ngroups), grp = (int)(item - (long long)t * a.ngroups);
+        const long long p = (long long)grp * 32 + lane, pc = p < a.plane ? p : a.plane - 1;
+        const char *wp = reinterpret_cast<const char *>(w + (npsf > 1 ? (t0 + t) * wstride : 0) + pc);
+        auto wrow = [&](int row) { return __ldg(reinterpret_cast<const float2 *>(wp + (unsigned)row * pb8)); };
+        const float g = a.fresp ? a.fresp[pc] : 1.f;
+        float2 v[N], e0, e1;
+#pragma unroll 1
+        for (int step = 0; step < 4; ++step) {
+            if (step < 2) {
+                pair_sync(pair);  // the buffer has been read
+                zf_generator<N>(v, step, half, wp, pb8, a, buf, pair);
+                if (step == 1) {
+                    pair_sync(pair);
+                    // the tile's planes, 16 bytes (two frequencies) per copy; past
+                    // the last frequency nothing (not stored either)
+                    const long long q = (long long)grp * 32 + 2 * (lane & 15);
+                    if (q < a.plane) {
+                        const float2 *src = S + (long long)t * Z * a.plane + q;
+                        for (int j = half * 2 + (lane >> 4); j < Z; j += 4)
+                            cp_async16(xbuf + j * 32 + 2 * (lane & 15), src + (long long)j * a.plane);
+                    }
+                }
+            } else if (step == 2) {
+                cp_async_wait();
+                pair_sync(pair);
+#pragma unroll
+                for (int j = 0; j < N; ++j) v[j] = j < LO || j < Z ? buf[j * 32] : make_float2(0.f, 0.f);
+                // the ends halved (planes past the last are zero)
+                e0 = pmul(v[0], 0.5f);
+                e1 = pmul(buf[(Z - 1) * 32], 0.5f);
+                v[0] = e0;
+#pragma unroll
+                for (int j = LO - 1; j < N; ++j) v[j] = pmul(v[j], j < Z - 1 ? 1.f : 0.5f);
+            }
+            if (half && step < 3) {
+#pragma unroll
+                for (int j = 1; j < N; ++j) v[j] = cmul(v[j], make_float2(unit_root<N>(j).x, -unit_root<N>(j).y));
+            }
+            zdft<N, false>(v);
+            if (step < 2) {
+                const float scale = g * (1.0f / (2 * N));
+                float2 *o = tab + step * N * 32;
+#pragma unroll
+                for (int k = 0; k < N; ++k) o[k * 32] = pmul(v[k], scale);
+            } else if (step == 2) {
+                if (half)
+                    zf_mix<N, true, 32>(v, tab, tab + N * 32);
+                else
+                    zf_mix<N, false, 32>(v, tab, tab + N * 32);
+            }
+        }
+        constexpr int M = 3 * N / 5;
+        pair_sync(pair);  // the planes have been read
+        if (half) {
+#pragma unroll
+            for (int i = 0; i < M; ++i)
+                buf[i * 32] = cmul(make_float2(unit_root<N>(i).x, unit_root<N>(i).y), make_float2(v[i].y, v[i].x));
+        } else {
+#pragma unroll
+            for (int i = M; i < N; ++i) buf[i * 32] = make_float2(v[i].y, v[i].x);
+        }
+        pair_sync(pair);
+        const float2 g0 = pmul(e0, g), g1 = pmul(e1, g);
+        char *yp = reinterpret_cast<char *>(S + (long long)t * Z * a.plane + pc);
+        auto finish = [&](int i, float2 y, float2 &near) {
+            if (a.far) {
+                const float2 next = wrow(i + Z);
+                y = cfma(g0, next, y);
+                y = cfma(g1, near, y);
+                near = next;
+            }
+            if (p < a.plane) *reinterpret_cast<float2 *>(yp + (unsigned)i * pb8) = y;
+        };
+        if (half) {
+            float2 near = a.far ? wrow(M + Z - 1) : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int i = M; i < N; ++i)
+                if (i < LO || i < Z)
+                    finish(i, cfma(make_float2(unit_root<N>(i).x, unit_root<N>(i).y), make_float2(v[i].y, v[i].x), buf[i * 32]),
+                           near);
+        } else {
+            float2 near = a.far ? wrow(Z - 1) : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < M; ++i) finish(i, padd(make_float2(v[i].y, v[i].x), buf[i * 32]), near);
+        }
+    }
+}
+
+template <int N>
+int zt_launch(float2 *S, const float2 *w, long long wstride, int t0, int npsf, const ZfArgs &args_in, cudaStream_t st) {
+    ZfArgs a = args_in;
+    const void *fn = (const void *)k_zfft_tiles<N>;
+    if (int rc = mm_set_smem(fn, zt_smem(N))) return rc;
+    a.ngroups = (int)((a.plane + 31) / 32);
+    const long long ctas = ((long long)a.ngroups * a.nt + zt_warps(N) / 2 - 1) / (zt_warps(N) / 2);
+    const int grid = ctas < mm_sm_count() ? (int)ctas : mm_sm_count();
+    void *args[] = {&S, &w, &wstride, &t0, &npsf, &a};
+    MM_CUDA_TRY(cudaLaunchKernel(fn, dim3(grid), dim3(zt_warps(N) * 32), args, zt_smem(N), st));
+    mm_launch_counter_add();
+    return MM_OK;
+}
+
 template <int N>
 int zf_launch(float2 *S, const float2 *w, const ZfArgs &args_in, cudaStream_t st) {
     ZfArgs a = args_in;
@@ -482,6 +620,28 @@ int mm_launch_zfft_apply(float2 *S, const float2 *w, int Z, int zpad, int Zp, lo
         case 45: return zf_launch<45>(S, w, a, st);
         case 56: return zf_launch<56>(S, w, a, st);
         case 50: return zf_launch<50>(S, w, a, st);
+    }
+    return MM_EINVAL;
+}
+
+int mm_launch_zfft_tiles(float2 *S, const float2 *w, long long wstride, int Z, int zpad, int Zp, long long plane, int t0,
+                         int nt, int npsf, const float *fresp, cudaStream_t st) {
+    MM_REQUIRE(Zp == Z + 2 * zpad && wstride % 2 == 0 && mm_zfft_supported(Z, zpad, nt, plane, w),
+               "z operator: depth %d, padding %d", Z, zpad);
+    ZfArgs a = {};
+    a.Z = Z;
+    a.Zp = Zp;
+    a.nt = nt;
+    a.far = zpad == Z - 1;
+    a.plane = plane;
+    a.fresp = fresp;
+    switch (zf_length(Z, zpad)) {
+        case 30: return zt_launch<30>(S, w, wstride, t0, npsf, a, st);
+        case 35: return zt_launch<35>(S, w, wstride, t0, npsf, a, st);
+        case 40: return zt_launch<40>(S, w, wstride, t0, npsf, a, st);
+        case 45: return zt_launch<45>(S, w, wstride, t0, npsf, a, st);
+        case 50: return zt_launch<50>(S, w, wstride, t0, npsf, a, st);
+        case 56: return zt_launch<56>(S, w, wstride, t0, npsf, a, st);
     }
     return MM_EINVAL;
 }

@@ -63,3 +63,30 @@ def test_short_transforms_at_the_edges_of_their_lengths(Z, near):
             err = (got[12] - want).abs().max() / want.abs().max()
             assert err < 2e-5, (ts, blur, float(err))
             assert torch.equal(got[4], got[12]) and torch.equal(got[6], got[12]), (ts, blur)
+
+
+@pytest.mark.parametrize("Z", [26, 31, 37, 39, 41, 46, 49, 51, 56])  # no multiples of 5: those have their own form
+@pytest.mark.parametrize("near", [False, True])
+def test_short_transforms_with_a_kernel_per_tile(Z, near):
+    """A PSF per tile at depths of every length: against the direct sum (2e-5 of
+    the largest voxel), planes that end inside a group of 32 frequencies, batches
+    past tile 0, and the same bits for every batch."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from mermake_gb300 import _lib, deconvolver, synth
+    if near and Z % 2:
+        pytest.skip("no such padding at an odd depth")
+    for ts, ov in ((14, 3), (30, 9)):
+        X, Y = 3 * ts - 1, 2 * ts
+        img = synth.hyb_stack(Z, X, Y, 40, seed=Z + ts).cuda()
+        psfs = {i: synth.gaussian_psf((5, 7, 7), 1.0 + 0.1 * i, 1.1 + 0.05 * i) for i in range(6)}
+        dec = deconvolver.Deconvolver(psfs, (Z, X, Y), tile_size=ts, zpad=(Z - 2) // 2 if near else Z - 1, overlap=ov,
+                                      beta=0.01)
+        for blur in (None, 6):
+            with _lib.blur_mode(_lib.MM_BLUR_EXACT if blur is None else _lib.MM_BLUR_SPECTRAL):
+                with _lib.zform(_lib.MM_ZFORM_DIRECT):
+                    want = dec.apply(img, None, blur_radius=blur)
+                got = {b: dec.apply(img, None, blur_radius=blur, batch=b) for b in (1, 4, 6)}
+            err = (got[6] - want).abs().max() / want.abs().max()
+            assert err < 2e-5, (ts, blur, float(err))
+            assert torch.equal(got[1], got[6]) and torch.equal(got[4], got[6]), (ts, blur)
